@@ -190,7 +190,10 @@ gs_status gs_rasterizer_set_lambda_dist(gs_rasterizer* r, float lambda_dist);
  * gs_rasterizer_check reports as GS_ERR_DEVICE_TIMEOUT; 0 gives up at once)
  * and drain_wait_cycles for the copies to land before an expired block exits
  * (at least 1e8 cycles, else GS_ERR_INVALID_ARG). Defaults 2e9 and 2e9 SM
- * cycles (about 1 s each at 1.965 GHz). Host-only; later steps use them. */
+ * cycles (about 1 s each at 1.965 GHz). A copy limit below 2e6 cycles also
+ * becomes the time a block of the handle's sorts waits for an earlier tile's
+ * counts before it counts that tile itself (results do not depend on it).
+ * Host-only; later steps use them. */
 gs_status gs_rasterizer_set_wait_limits(gs_rasterizer* r, uint64_t copy_wait_cycles, uint64_t drain_wait_cycles);
 /* Rasterizer::forward (rasterizer.rs:389-448): projection, binning, forward
  * raster for n_views cameras (1 = the reference's single-view call). */
@@ -447,8 +450,7 @@ gs_status gs_binner_buffer(gs_binner* b, uint32_t which, void** dptr, size_t* by
  * Both take caller device pointers. The scan's scratch is allocated on first
  * use; the sort takes its own from a memory pool of the library in stream
  * order, which keeps up to 512 MiB between calls (both held until
- * gs_shutdown). A sort of more than 8192 pairs contains bounded waits between
- * its blocks; GS_ERR_DEVICE_TIMEOUT when one expires (contents undefined). */
+ * gs_shutdown). */
 gs_status gs_radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, uint32_t key_bits, void* stream);
 gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev, void* stream);
 
@@ -464,8 +466,7 @@ gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, u
  * it before any stream capture, and do not call this entry point after
  * resetting the device (cudaDeviceReset), which invalidates that address.
  * Calls share the array: calls that overlap on the GPU (different streams,
- * or different host threads) race and corrupt each other's results, or wait
- * for one another until a bounded wait (about a second) gives up.
+ * or different host threads) race and corrupt each other's results.
  * Stream-ordered, does not synchronise. */
 gs_status gs_radix_sort_pairs_noalloc(uint32_t* keys, uint32_t* vals, uint64_t n, uint32_t key_bits, void* stream);
 

@@ -416,13 +416,13 @@ gs_status run_forward(gs_rasterizer* r, const ViewInfo* vdev, const ViewInfo* vh
   // the entry scan and the expansion read them sequentially.
   TRY_LAUNCH(r, launch_sort_reset(r->sort, st));
   TRY_LAUNCH(r, launch_radix_sort(r->item_keys[0], r->item_vals[0], r->item_keys[1], r->item_vals[1], items, nullptr,
-                                  32, r->sort, 0, &in1, st, r->words + 1, r->counts, r->sorted_counts));
+                                  32, r->sort, 0, &in1, st, r->counts, r->sorted_counts));
   uint32_t* perm = r->item_vals[in1];
   uint32_t* n_entries = r->words;  // u32 saturated
   EntryScanArgs sa{};
   sa.in = r->sorted_counts; sa.out = r->offsets; sa.n_host = items;
   sa.total_u32 = n_entries; sa.total_u64 = r->entry_total; sa.capacity = r->max_entries;
-  sa.error_word = r->words + 1; sa.sort_hdr = r->sort.hdr[0];
+  sa.error_word = r->words + 1;
   TRY_LAUNCH(r, launch_entry_scan(sa, r->sort, 0, st));
   mark(prof, 1, st);
   ExpandArgs ea{};
@@ -454,9 +454,9 @@ gs_status run_forward(gs_rasterizer* r, const ViewInfo* vdev, const ViewInfo* vh
   // The tile sort's final pass also records each tile's range; the fix-up
   // turns it into [start, end).
   TRY_LAUNCH(r, launch_radix_sort_pairs(r->ent_pairs[0], r->ent_pairs[1], r->max_entries, n_entries, bits, r->sort, 1,
-                                        &r->ent_in1, st, r->words + 1, r->ranges, (uint32_t)tiles, true));
+                                        &r->ent_in1, st, r->ranges, (uint32_t)tiles, true));
   mark(prof, 3, st);
-  TRY_LAUNCH(r, launch_ranges_fix(r->ranges, (uint32_t)tiles, r->sort, 1, st));
+  TRY_LAUNCH(r, launch_ranges_fix(r->ranges, (uint32_t)tiles, st));
   r->order_valid = persistent;
   if (persistent) TRY_LAUNCH(r, launch_tile_order(r->ranges, nullptr, (uint32_t)tiles, r->tile_order, st));
   mark(prof, 4, st);
@@ -514,13 +514,12 @@ gs_status run_forward(gs_rasterizer* r, const ViewInfo* vdev, const ViewInfo* vh
     mark(prof, 2, st);
     int in1b = 0;
     TRY_LAUNCH(r, launch_radix_sort_pairs(r->ent_pairs[0], r->ent_pairs[1], r->max_entries, r->cutw + 2, bits, r->sort,
-                                          1, &in1b, st, r->words + 1, r->ranges, (uint32_t)tiles, false,
-                                          r->entry_total));
+                                          1, &in1b, st, r->ranges, (uint32_t)tiles, false, r->entry_total));
     if (in1b != r->ent_in1) return fail(r, GS_ERR_STATE, "completion sort ended in the other buffer");
     mark(prof, 3, st);
     TRY_LAUNCH(r, launch_ranges_fix_list(r->inc_list, r->cutw, r->ranges, (uint32_t)tiles, r->entry_total,
                                          r->entry_total2, r->gmask_valid ? r->gmask : nullptr, r->inc_skip,
-                                         r->inc_src, r->sort, 1, st));
+                                         r->inc_src, st));
     mark(prof, 4, st);
     RasterArgs rb = ra;
     rb.cut_pass = 2;
@@ -969,9 +968,6 @@ gs_status gs_rasterizer_create(const gs_raster_config* cfg_in, gs_rasterizer** o
   if (e == cudaSuccess) e = cudaMemset(r->accum_norm, 0, sizeof(float) * N);
   if (e == cudaSuccess && r->cut_on) e = cudaMemset(r->tile_cut, 0xff, sizeof(uint32_t) * (size_t)r->max_tiles);
   if (e == cudaSuccess && r->cut_on) e = cudaMemset(r->cutw, 0, sizeof(uint32_t) * 4);
-  // a depth order that a sort gave up on still holds valid items
-  for (int k = 0; k < 2; ++k)
-    if (e == cudaSuccess) e = cudaMemset(r->item_vals[k], 0, sizeof(uint32_t) * I);
   if (e != cudaSuccess) return bail(e, "initial memset");
   *out = r;
   return GS_OK;
@@ -1049,6 +1045,7 @@ gs_status gs_rasterizer_set_wait_limits(gs_rasterizer* r, uint64_t copy_wait_cyc
     return fail(r, GS_ERR_INVALID_ARG, "drain wait below 1e8 cycles, or a limit beyond 2^62");
   r->wait_cycles[0] = (long long)copy_wait_cycles;
   r->wait_cycles[1] = (long long)drain_wait_cycles;
+  r->sort.wait_cycles = std::min(SORT_WAIT_CYCLES, r->wait_cycles[0]);
   return GS_OK;
 }
 
@@ -1716,8 +1713,6 @@ static gs_status mcmc_ready(gs_rasterizer* r, cudaStream_t st) {
   if (r->mcmc_u32) return GS_OK;
   const size_t N = r->cap;
   TRY_CUDA(r, dalloc(r->mcmc_u32, 19 * N));
-  // sorted indices stay in range even when a sort gives up
-  TRY_CUDA(r, cudaMemsetAsync(r->mcmc_u32, 0, sizeof(uint32_t) * 19 * N, st));
   TRY_CUDA(r, dalloc(r->mcmc_u64, 2 * N + 1));
   TRY_CUDA(r, dalloc(r->mcmc_jump, 64 * (size_t)MCMC_JUMP_LEVELS));
   TRY_CUDA(r, dalloc(r->mcmc_rng, 1));
@@ -1752,7 +1747,6 @@ gs_status gs_mcmc_relocate(gs_rasterizer* r, const gs_mcmc_config* c, uint32_t n
   if (s) return s;
   const size_t N = r->cap;
   McmcArgs a{};
-  a.error_word = r->words + 1;
   a.n = n; a.dead_threshold = c->dead_threshold; a.split_ratio = c->split_ratio;
   a.jump = r->mcmc_jump; a.rng_state = r->mcmc_rng; a.counters = r->mcmc_counters;
   uint32_t* u = r->mcmc_u32;
@@ -1899,10 +1893,10 @@ extern "C" gs_status gs_binner_encode(gs_binner* b, const uint32_t* rects_dev, c
   if (!e) e = launch_entry_scan(sa, b->sort, 1, st);
   int in1 = 0;
   if (!e) e = launch_radix_sort(b->item_keys[0], b->item_vals[0], b->item_keys[1], b->item_vals[1], n, nullptr, 32,
-                                b->sort, 0, &in1, st, b->words + 1, b->counts, b->sorted_counts);
+                                b->sort, 0, &in1, st, b->counts, b->sorted_counts);
   uint32_t* perm = b->item_vals[in1];
   sa.in = b->sorted_counts; sa.out = b->offsets; sa.total_u32 = b->words; sa.total_u64 = b->total;
-  sa.capacity = b->max_entries; sa.sort_hdr = b->sort.hdr[0];
+  sa.capacity = b->max_entries;
   if (!e) e = launch_entry_scan(sa, b->sort, 0, st);
   if (!e) {
     ExpandArgs ea{};
@@ -1918,9 +1912,9 @@ extern "C" gs_status gs_binner_encode(gs_binner* b, const uint32_t* rects_dev, c
   }
   int ent_in1 = 0;
   if (!e) e = launch_radix_sort_pairs(b->ent_pairs[0], b->ent_pairs[1], b->max_entries, b->words,
-                                      tile_key_bits(b->num_tiles), b->sort, 1, &ent_in1, st, b->words + 1, b->ranges,
-                                      b->num_tiles, true, nullptr, b->sorted_entries);
-  if (!e) e = launch_ranges_fix(b->ranges, b->num_tiles, b->sort, 1, st);
+                                      tile_key_bits(b->num_tiles), b->sort, 1, &ent_in1, st, b->ranges, b->num_tiles,
+                                      true, nullptr, b->sorted_entries);
+  if (!e) e = launch_ranges_fix(b->ranges, b->num_tiles, st);
   if (e) return fail(nullptr, GS_ERR_CUDA, std::string("binner encode: ") + cudaGetErrorString((cudaError_t)e));
   // The reference asserts on overflow; report it here (blocking).
   uint32_t w = 0;
@@ -2017,21 +2011,17 @@ extern "C" gs_status gs_radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_
   uint32_t* k1 = reinterpret_cast<uint32_t*>(buf);
   uint32_t* v1 = reinterpret_cast<uint32_t*>(buf + arr);
   const SortScratch sc = sort_scratch(buf + 2 * arr, n, 0);
-  uint32_t aborted = 0;
   int in1 = 0;
   int le = launch_sort_reset(sc, st);
-  if (!le) le = launch_radix_sort(keys, vals, k1, v1, n, nullptr, (int)key_bits, sc, 0, &in1, st, sc.hdr[1]);
+  if (!le) le = launch_radix_sort(keys, vals, k1, v1, n, nullptr, (int)key_bits, sc, 0, &in1, st);
   if (!le && in1) {  // an odd number of passes ends in the ping-pong buffers
     le = (int)cudaMemcpyAsync(keys, k1, n * 4, cudaMemcpyDeviceToDevice, st);
     if (!le) le = (int)cudaMemcpyAsync(vals, v1, n * 4, cudaMemcpyDeviceToDevice, st);
   }
-  if (!le && n > (uint64_t)RS_SMALL)  // (the single-block sort waits for nothing)
-    le = (int)cudaMemcpyAsync(&aborted, sc.hdr[1], 4, cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(buf, st);
   if (le) return fail(nullptr, GS_ERR_CUDA, cudaGetErrorString((cudaError_t)le));
   const cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(nullptr, GS_ERR_CUDA, cudaGetErrorString(e));
-  if (aborted) return fail(nullptr, GS_ERR_DEVICE_TIMEOUT, "a bounded device wait expired");
   return GS_OK;
 }
 

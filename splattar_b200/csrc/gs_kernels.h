@@ -205,7 +205,10 @@ struct SortScratch {
   size_t state_words;  // of one set
   size_t reset_bytes;
   bool wide;
+  // A sort's block that has waited this many cycles for a tile counts it itself.
+  long long wait_cycles;
 };
+constexpr long long SORT_WAIT_CYCLES = 2000000;  // about a millisecond
 constexpr size_t sort_scan_words(uint64_t scan_n) { return (size_t)((scan_n + ES_TILE - 1) / ES_TILE + 1); }
 constexpr size_t sort_state_words(uint64_t max_n) { return (size_t)((max_n + RS_TILE - 1) / RS_TILE + 1) * 256; }
 constexpr bool sort_wide(uint64_t max_n) { return max_n >= (1ull << 30); }
@@ -228,14 +231,14 @@ inline SortScratch sort_scratch(void* base, uint64_t max_n, uint64_t scan_n) {
   s.state_words = sort_state_words(max_n);
   s.reset_bytes = sort_reset_bytes(scan_n);
   s.wide = sort_wide(max_n);
+  s.wait_cycles = SORT_WAIT_CYCLES;
   return s;
 }
 int launch_sort_reset(const SortScratch& sc, cudaStream_t st);
 
 // Exclusive scan of item counts in one pass, with the entry-capacity guard
 // (capacity 0: none): when *base + total > capacity, ERR_ENTRY_CAPACITY is
-// flagged and the totals are zero. sort_hdr: the header of the sort that
-// ordered the items; when that sort gave up, the totals are zero.
+// flagged and the totals are zero.
 struct EntryScanArgs {
   const uint32_t* in;
   const uint32_t* perm;
@@ -247,7 +250,6 @@ struct EntryScanArgs {
   const unsigned long long* base;
   uint64_t capacity;
   uint32_t* error_word;
-  const uint32_t* sort_hdr;
 };
 int launch_entry_scan(const EntryScanArgs& a, const SortScratch& sc, int which, cudaStream_t st);
 
@@ -255,26 +257,24 @@ int launch_entry_scan(const EntryScanArgs& a, const SortScratch& sc, int which, 
 // `hdr` of the scratch (cleared since its last use). Ping-pongs between
 // (k0,v0) and (k1,v1); returns in *result_in_1 where the output is. With
 // gather_dst, the final pass also writes gather_dst[i] = gather_src[val] for
-// every sorted position i. A wait that expires sets ERR_TIMEOUT in
-// *error_word (when non-null) and the header's abort word; the output is then
-// undefined.
+// every sorted position i.
 int launch_radix_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint64_t n_host, const uint32_t* n_dev,
                       int key_bits, const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st,
-                      uint32_t* error_word, const uint32_t* gather_src = nullptr, uint32_t* gather_dst = nullptr);
+                      const uint32_t* gather_src = nullptr, uint32_t* gather_dst = nullptr);
 // The same sort on interleaved (key, val) pairs, ping-ponging between p0 and p1.
 // With `ranges` (zero-filled, by this call with zero_ranges; num_ranges
 // entries) the sort's final pass also records each key's output range;
 // launch_ranges_fix then converts it to [start, end) per key ((0, 0) for
-// absent keys, and for all keys when the sort gave up) — the tile ranges
-// without a separate pass over the sorted entries. With `base` (device), the
+// absent keys) — the tile ranges without a separate pass over the sorted
+// entries. With `base` (device), the
 // sort covers elements [*base, *base + n) of both buffers and the recorded
 // ranges are positions in the whole buffer. With `values`, the final pass
 // writes the sorted values there and no pairs.
 int launch_radix_sort_pairs(uint2* p0, uint2* p1, uint64_t n_host, const uint32_t* n_dev, int key_bits,
-                            const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st, uint32_t* error_word,
-                            uint2* ranges, uint32_t num_ranges, bool zero_ranges,
-                            const unsigned long long* base = nullptr, uint32_t* values = nullptr);
-int launch_ranges_fix(uint2* ranges, uint32_t num_tiles, const SortScratch& sc, int hdr, cudaStream_t st);
+                            const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st, uint2* ranges,
+                            uint32_t num_ranges, bool zero_ranges, const unsigned long long* base = nullptr,
+                            uint32_t* values = nullptr);
+int launch_ranges_fix(uint2* ranges, uint32_t num_tiles, cudaStream_t st);
 // Tile order for the persistent raster kernels: tiles bucketed by the
 // logarithm of their work (four buckets per octave; the work is lengths[t]
 // when given, else the tile's entry count), heaviest bucket first. Order
@@ -346,8 +346,7 @@ int launch_ranges_reset_list(const uint32_t* list, const uint32_t* count, uint2*
 // gmask[src[i]] to the tile's new start.
 int launch_ranges_fix_list(const uint32_t* list, const uint32_t* count, uint2* ranges, uint32_t max_list,
                            unsigned long long* entry_total, const unsigned long long* total2, uint8_t* gmask,
-                           const uint32_t* skip, const uint32_t* src, const SortScratch& sc, int hdr,
-                           cudaStream_t st);
+                           const uint32_t* skip, const uint32_t* src, cudaStream_t st);
 // mask_off[t] = Σ_{t' < t} ⌈len(t')/32⌉ over the tiles' entry ranges.
 int launch_mask_offsets(const uint2* ranges, uint32_t num_tiles, uint32_t* words, uint32_t* mask_off, void* scratch,
                         cudaStream_t st);
@@ -413,7 +412,6 @@ int launch_densify(DensifyArgs& a, void* scan_scratch, cudaStream_t st);
 // ---- MCMC relocation and noise (gs_mcmc.cu) ----
 constexpr int MCMC_JUMP_LEVELS = 33;  // powers M^(2^j) of the xorshift64 step, j < 33
 struct McmcArgs {
-  uint32_t* error_word;  // ERR_TIMEOUT when a sort's bounded wait expires
   uint32_t n;
   float dead_threshold, split_ratio;
   const uint64_t* jump;          // MCMC_JUMP_LEVELS × 64 rows

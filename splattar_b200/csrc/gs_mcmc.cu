@@ -354,7 +354,7 @@ int launch_mcmc_relocate(McmcArgs& a, int prec, void* scan_scratch, const SortSc
   if (a.split_ratio > 0.f) {
     int in1 = 0;
     e = launch_sort_reset(sc, st);
-    if (!e) e = launch_radix_sort(a.size_key, a.size_val, a.key2, a.val2, a.n, nullptr, 32, sc, 0, &in1, st, a.error_word);
+    if (!e) e = launch_radix_sort(a.size_key, a.size_val, a.key2, a.val2, a.n, nullptr, 32, sc, 0, &in1, st);
     if (e) return e;
     a.sorted_size_key = in1 ? a.key2 : a.size_key;
     k_mcmc_over_flags<<<g, 256, 0, st>>>(a);
@@ -362,7 +362,7 @@ int launch_mcmc_relocate(McmcArgs& a, int prec, void* scan_scratch, const SortSc
     if (e) return e;
     k_mcmc_over_list<<<g, 256, 0, st>>>(a);
     // The size keys are consumed; their buffers take the second sort.
-    e = launch_radix_sort(a.over_key, a.over_val, a.key2, a.val2, a.n, a.counters + 5, 32, sc, 1, &in1, st, a.error_word);
+    e = launch_radix_sort(a.over_key, a.over_val, a.key2, a.val2, a.n, a.counters + 5, 32, sc, 1, &in1, st);
     if (e) return e;
     a.over_sorted_val = in1 ? a.val2 : a.over_val;
     e = launch_scan(a.leftover_flag, nullptr, a.left_rank, a.n, a.counters + 0, a.counters + 6, nullptr, scan_scratch,

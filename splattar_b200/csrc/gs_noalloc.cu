@@ -88,7 +88,7 @@ extern "C" gs_status gs_radix_sort_pairs_noalloc(uint32_t* keys, uint32_t* vals,
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int in1 = 0;
   int le = launch_sort_reset(sc, st);
-  if (!le) le = launch_radix_sort(keys, vals, k1, v1, n, nullptr, (int)key_bits, sc, 0, &in1, st, nullptr);
+  if (!le) le = launch_radix_sort(keys, vals, k1, v1, n, nullptr, (int)key_bits, sc, 0, &in1, st);
   if (!le && in1) {
     le = (int)cudaMemcpyAsync(keys, k1, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
     if (!le) le = (int)cudaMemcpyAsync(vals, v1, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);

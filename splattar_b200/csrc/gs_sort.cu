@@ -19,9 +19,10 @@
 // its counts and sums the tiles before it by looking back at their published
 // counts (the single-pass scan of Merrill and Garland 2016; applied to radix
 // passes by Adinets and Merrill, "Onesweep", 2022). A block only ever waits
-// for tiles with lower tickets, which are running or done, and every wait is
-// bounded: after WAIT_CYCLES the sort flags ERR_TIMEOUT and its remaining
-// blocks leave; the entry scan and the range fix-up then publish no entries.
+// for tiles with lower tickets, which are running or done. A sort's waits are
+// bounded and end in the same result: a block that has waited long enough for
+// a tile counts that tile itself, from the pass's input, which nothing writes
+// meanwhile.
 #include <algorithm>
 
 #include <cub/block/block_reduce.cuh>
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, 
 // Words of a sort's or scan's header (zeroed by launch_sort_reset).
 constexpr int SH_HIST = 0;        // [4][256] digit counts of all passes
 constexpr int SH_TICKET = 1024;   // [4] tile tickets, one per pass
-constexpr int SH_ABORT = 1028;    // a bounded wait of this sort expired
+constexpr int SH_ABORT = 1028;    // a bounded wait of this scan expired
 static_assert(SH_ABORT < SORT_HDR_WORDS, "header words");
 
 constexpr long long WAIT_CYCLES = 2000000000ll;  // about a second
@@ -146,10 +147,11 @@ __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long 
 // Sum of everything before tile t in the column of published words at
 // `col` (stride `stride` words per tile), t > 0. LB predecessors are read at
 // once, so a chain of tiles that published only their own counts costs one
-// memory latency per LB tiles. False when the wait expired.
-template <typename W>
-__device__ __forceinline__ bool look_back(const W* col, uint32_t stride, uint32_t t, const uint32_t* abort_word,
-                                          W& sum_out) {
+// memory latency per LB tiles. After `wait` cycles without the next tile's
+// word, `recount` (tile -> its own count) takes its place: the sum is the
+// same, and the loop ends whatever the other blocks do.
+template <typename W, class F>
+__device__ __forceinline__ W look_back(const W* col, uint32_t stride, uint32_t t, long long wait, F&& recount) {
   using P = Published<W>;
   constexpr int LB = 8;
   W sum = 0;
@@ -170,7 +172,7 @@ __device__ __forceinline__ bool look_back(const W* col, uint32_t stride, uint32_
         } else {
           sum += v[k] & P::VALUE;
           ++used;
-          if (v[k] & P::PREFIX) { sum_out = sum; return true; }
+          if (v[k] & P::PREFIX) return sum;
         }
       }
     }
@@ -178,7 +180,11 @@ __device__ __forceinline__ bool look_back(const W* col, uint32_t stride, uint32_
     if (stop && used == 0) {
       const long long now = clock64();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > WAIT_CYCLES || ld_relaxed(abort_word)) return false;
+      if (now - t0 >= wait) {
+        sum += recount(left - 1);
+        --left;
+        t0 = 0;
+      }
     } else {
       t0 = 0;
     }
@@ -306,6 +312,17 @@ __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, 
   }
 }
 
+// How many of a whole tile's keys have this digit (look_back's recount). Not
+// inlined: it is hardly ever called, and the passes are short of registers
+// (sort of 4 million pairs 223 us without it, 220 with).
+template <class IO>
+__device__ __noinline__ uint32_t count_digit(IO io, uint64_t tile, int shift, uint32_t mask, uint32_t digit) {
+  uint32_t c = 0;
+#pragma unroll 8
+  for (int i = 0; i < RS_TILE; ++i) c += ((io.key(tile * RS_TILE + i) >> shift) & mask) == digit;
+  return c;
+}
+
 // ranges (final pass of a key sort only, else null): every run of one key
 // inside a staged tile is folded into that key's output range, stored as
 // (~first position, one past the last position) with atomicMax on both, so
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
                                                                  int pass, int shift, int nbits, uint32_t* hdr,
                                                                  W* state, W* next_state, uint2* ranges,
                                                                  uint32_t num_ranges, const unsigned long long* base,
-                                                                 uint32_t* error_word) {
+                                                                 long long wait) {
   using P = Published<W>;
   __shared__ uint2 s_e[RS_TILE];
   __shared__ uint16_t s_wh[RS_WARPS][RS_BINS];
@@ -392,19 +409,14 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
       }
     }
     W before = 0;
-    bool ok = true;
     if (t > 0 && tid <= (int)mask) {
-      ok = look_back<W>(state + tid, RS_BINS, t, hdr + SH_ABORT, before);
-      if (ok) st_relaxed(mine, P::PREFIX | (before + (W)cnt));
+      before = look_back(state + tid, RS_BINS, t, wait, [&](uint32_t tile) {
+        return (W)count_digit(io, tile, shift, mask, (uint32_t)tid);
+      });
+      st_relaxed(mine, P::PREFIX | (before + (W)cnt));
     }
     if (tid < RS_BINS) s_gofs[tid] = digit_base + (uint32_t)before - excl;  // output position = s_gofs[d] + position in the tile
-    if (!__syncthreads_and(ok)) {
-      if (tid == 0) {
-        st_relaxed(hdr + SH_ABORT, 1u);
-        if (error_word != nullptr) atomicOr(error_word, ERR_TIMEOUT);
-      }
-      return;
-    }
+    __syncthreads();
 #pragma unroll 4
     for (int i = tid; i < tn; i += RS_THREADS) {
       const uint2 v = s_e[i];
@@ -513,8 +525,7 @@ __global__ void __launch_bounds__(ES_THREADS) k_entry_scan(EntryScanArgs a, uint
   __shared__ unsigned long long s_before;
   __shared__ uint32_t s_tile;
   const int tid = threadIdx.x, lane = tid & 31;
-  const bool bad = a.sort_hdr != nullptr && a.sort_hdr[SH_ABORT] != 0u;  // the order was never written
-  const uint64_t n = bad ? 0 : read_n(a.n_host, a.n_dev);
+  const uint64_t n = read_n(a.n_host, a.n_dev);
   const uint32_t tiles = n ? (uint32_t)((n + ES_TILE - 1) / ES_TILE) : 1u;
   auto finish = [&](unsigned long long total) {
     if (a.capacity && (a.base != nullptr ? *a.base : 0ull) + total > a.capacity) {
@@ -818,15 +829,13 @@ __global__ void __launch_bounds__(256) k_ranges_reset_list(const uint32_t* list,
 __global__ void __launch_bounds__(256) k_ranges_fix_list(const uint32_t* list, const uint32_t* count, uint2* ranges,
                                                          uint32_t max_list, unsigned long long* entry_total,
                                                          const unsigned long long* total2, uint8_t* gmask,
-                                                         const uint32_t* skip, const uint32_t* src,
-                                                         const uint32_t* hdr) {
+                                                         const uint32_t* skip, const uint32_t* src) {
   const uint32_t m = min(*count, max_list);
-  const bool bad = hdr[SH_ABORT] != 0u;  // the completion sort gave up
   for (uint32_t i = blockIdx.x; i < m; i += gridDim.x) {
     const uint32_t t = list[i];
     const uint2 r = ranges[t];
     __syncthreads();  // every thread holds the recorded range before it is replaced
-    const uint2 f = r.y && !bad ? make_uint2(~r.x, r.y) : make_uint2(0u, 0u);
+    const uint2 f = r.y ? make_uint2(~r.x, r.y) : make_uint2(0u, 0u);
     if (threadIdx.x == 0) ranges[t] = f;
     if (gmask != nullptr) {
       const uint32_t sk = skip[i], from = src[i];
@@ -883,7 +892,7 @@ namespace {
 
 template <class IO, typename W, class SWAP>
 int radix_passes(IO io, uint64_t n_host, const uint32_t* n_dev, int key_bits, const SortScratch& sc, int hdr,
-                 int* result_in_1, cudaStream_t st, uint32_t* error_word, SWAP swap, uint2* ranges = nullptr,
+                 int* result_in_1, cudaStream_t st, SWAP swap, uint2* ranges = nullptr,
                  uint32_t num_ranges = 0, const unsigned long long* base = nullptr, bool zero_ranges = false) {
   const int passes = (key_bits + 7) / 8, dbits = (key_bits + passes - 1) / passes;
   uint32_t* h = sc.hdr[hdr];
@@ -896,7 +905,7 @@ int radix_passes(IO io, uint64_t n_host, const uint32_t* n_dev, int key_bits, co
     const bool last = p + 1 == passes;
     k_rs_pass<IO, W><<<grid, RS_THREADS, 0, st>>>(last ? io : io.plain(), n_host, n_dev, p, shift, nbits, h,
                                                   state[p & 1], last ? nullptr : state[(p + 1) & 1],
-                                                  last ? ranges : nullptr, num_ranges, base, error_word);
+                                                  last ? ranges : nullptr, num_ranges, base, sc.wait_cycles);
     swap(io);
   }
   *result_in_1 = passes & 1;
@@ -918,7 +927,7 @@ int launch_small(const SplitIO& io, int n, int passes, int dbits, int key_bits, 
 
 int launch_radix_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uint64_t n_host, const uint32_t* n_dev,
                       int key_bits, const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st,
-                      uint32_t* error_word, const uint32_t* gather_src, uint32_t* gather_dst) {
+                      const uint32_t* gather_src, uint32_t* gather_dst) {
   SplitIO io{k0, v0, k1, v1, gather_src, gather_dst};
   if (n_host <= (uint64_t)RS_SMALL && n_dev == nullptr) {  // one launch, 26 us at 3000 pairs; 6 launches take 37 us at 16 thousand
     if (n_host == 0) { *result_in_1 = ((key_bits + 7) / 8) & 1; return 0; }
@@ -934,24 +943,23 @@ int launch_radix_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, ui
     x = y;
   };
   if (sc.wide)
-    return radix_passes<SplitIO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, error_word, swap);
-  return radix_passes<SplitIO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, error_word, swap);
+    return radix_passes<SplitIO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap);
+  return radix_passes<SplitIO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap);
 }
 
 int launch_radix_sort_pairs(uint2* p0, uint2* p1, uint64_t n_host, const uint32_t* n_dev, int key_bits,
-                            const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st, uint32_t* error_word,
-                            uint2* ranges, uint32_t num_ranges, bool zero_ranges, const unsigned long long* base,
-                            uint32_t* values) {
+                            const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st, uint2* ranges,
+                            uint32_t num_ranges, bool zero_ranges, const unsigned long long* base, uint32_t* values) {
   PairIO io{p0, p1, values};
   auto swap = [](PairIO& x) {
     PairIO y{x.out, const_cast<uint2*>(x.in), x.values};
     x = y;
   };
   if (sc.wide)
-    return radix_passes<PairIO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, error_word,
-                                                    swap, ranges, num_ranges, base, zero_ranges);
-  return radix_passes<PairIO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, error_word, swap,
-                                        ranges, num_ranges, base, zero_ranges);
+    return radix_passes<PairIO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges,
+                                                    num_ranges, base, zero_ranges);
+  return radix_passes<PairIO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges, num_ranges,
+                                        base, zero_ranges);
 }
 
 int launch_expand(const ExpandArgs& a, cudaStream_t st) {
@@ -989,21 +997,18 @@ int launch_ranges_reset_list(const uint32_t* list, const uint32_t* count, uint2*
 
 int launch_ranges_fix_list(const uint32_t* list, const uint32_t* count, uint2* ranges, uint32_t max_list,
                            unsigned long long* entry_total, const unsigned long long* total2, uint8_t* gmask,
-                           const uint32_t* skip, const uint32_t* src, const SortScratch& sc, int hdr,
-                           cudaStream_t st) {
-  k_ranges_fix_list<<<148, 256, 0, st>>>(list, count, ranges, max_list, entry_total, total2, gmask, skip, src,
-                                         sc.hdr[hdr]);
+                           const uint32_t* skip, const uint32_t* src, cudaStream_t st) {
+  k_ranges_fix_list<<<148, 256, 0, st>>>(list, count, ranges, max_list, entry_total, total2, gmask, skip, src);
   return (int)cudaGetLastError();
 }
 
 namespace {
 // (~first, end) from the final sort pass → [first, end); (0, 0) for a key no
 // element carried.
-__global__ void __launch_bounds__(256) k_ranges_fix(uint2* ranges, uint32_t num_tiles, const uint32_t* hdr) {
-  const bool bad = hdr[SH_ABORT] != 0u;  // the tile sort gave up: no tile has entries
+__global__ void __launch_bounds__(256) k_ranges_fix(uint2* ranges, uint32_t num_tiles) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < num_tiles; t += gridDim.x * blockDim.x) {
     const uint2 r = ranges[t];
-    ranges[t] = r.y && !bad ? make_uint2(~r.x, r.y) : make_uint2(0u, 0u);
+    ranges[t] = r.y ? make_uint2(~r.x, r.y) : make_uint2(0u, 0u);
   }
 }
 
@@ -1015,9 +1020,9 @@ __global__ void __launch_bounds__(256) k_tile_words(const uint2* ranges, uint32_
 }
 }  // namespace
 
-int launch_ranges_fix(uint2* ranges, uint32_t num_tiles, const SortScratch& sc, int hdr, cudaStream_t st) {
+int launch_ranges_fix(uint2* ranges, uint32_t num_tiles, cudaStream_t st) {
   if (num_tiles == 0) return 0;
-  k_ranges_fix<<<grid_for(num_tiles, 256, 148 * 8), 256, 0, st>>>(ranges, num_tiles, sc.hdr[hdr]);
+  k_ranges_fix<<<grid_for(num_tiles, 256, 148 * 8), 256, 0, st>>>(ranges, num_tiles);
   return (int)cudaGetLastError();
 }
 
