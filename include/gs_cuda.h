@@ -191,8 +191,9 @@ gs_status gs_rasterizer_set_lambda_dist(gs_rasterizer* r, float lambda_dist);
  * and drain_wait_cycles for the copies to land before an expired block exits
  * (at least 1e8 cycles, else GS_ERR_INVALID_ARG). Defaults 2e9 and 2e9 SM
  * cycles (about 1 s each at 1.965 GHz). A copy limit below 2e6 cycles also
- * becomes the time a block of the handle's sorts waits for an earlier tile's
- * counts before it counts that tile itself (results do not depend on it).
+ * becomes the time a block of the handle's sorts and entry scans waits for an
+ * earlier tile's counts before it counts that tile itself (results do not
+ * depend on it).
  * Host-only; later steps use them. */
 gs_status gs_rasterizer_set_wait_limits(gs_rasterizer* r, uint64_t copy_wait_cycles, uint64_t drain_wait_cycles);
 /* Rasterizer::forward (rasterizer.rs:389-448): projection, binning, forward

@@ -1925,10 +1925,6 @@ extern "C" gs_status gs_binner_encode(gs_binner* b, const uint32_t* rects_dev, c
     cudaMemset(b->words + 1, 0, 4);
     return fail(nullptr, GS_ERR_CAPACITY, "tile entries exceeded max_entries");
   }
-  if (w & ERR_TIMEOUT) {
-    cudaMemset(b->words + 1, 0, 4);
-    return fail(nullptr, GS_ERR_DEVICE_TIMEOUT, "a bounded device wait expired");
-  }
   return GS_OK;
 }
 

@@ -205,7 +205,7 @@ struct SortScratch {
   size_t state_words;  // of one set
   size_t reset_bytes;
   bool wide;
-  // A sort's block that has waited this many cycles for a tile counts it itself.
+  // A block that has waited this many cycles for a tile counts it itself.
   long long wait_cycles;
 };
 constexpr long long SORT_WAIT_CYCLES = 2000000;  // about a millisecond

@@ -19,7 +19,7 @@
 // its counts and sums the tiles before it by looking back at their published
 // counts (the single-pass scan of Merrill and Garland 2016; applied to radix
 // passes by Adinets and Merrill, "Onesweep", 2022). A block only ever waits
-// for tiles with lower tickets, which are running or done. A sort's waits are
+// for tiles with lower tickets, which are running or done. The waits are
 // bounded and end in the same result: a block that has waited long enough for
 // a tile counts that tile itself, from the pass's input, which nothing writes
 // meanwhile.
@@ -113,10 +113,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, 
 // Words of a sort's or scan's header (zeroed by launch_sort_reset).
 constexpr int SH_HIST = 0;        // [4][256] digit counts of all passes
 constexpr int SH_TICKET = 1024;   // [4] tile tickets, one per pass
-constexpr int SH_ABORT = 1028;    // a bounded wait of this scan expired
-static_assert(SH_ABORT < SORT_HDR_WORDS, "header words");
-
-constexpr long long WAIT_CYCLES = 2000000000ll;  // about a second
+static_assert(SH_TICKET + 4 <= SORT_HDR_WORDS, "header words");
 
 // A published count: the state in the top two bits, the value below. Flag and
 // value travel in one word, so relaxed accesses suffice.
@@ -518,7 +515,8 @@ __global__ void __launch_bounds__(NT) k_rs_small(SplitIO io, int n, int passes, 
 // than were allocated (base + total > capacity), the totals are set to zero
 // so that no later pass reads an entry that was never written.
 constexpr int ES_THREADS = 256, ES_ITEMS = ES_TILE / ES_THREADS;
-__global__ void __launch_bounds__(ES_THREADS) k_entry_scan(EntryScanArgs a, uint32_t* hdr, unsigned long long* state) {
+__global__ void __launch_bounds__(ES_THREADS) k_entry_scan(EntryScanArgs a, uint32_t* hdr, unsigned long long* state,
+                                                           long long wait) {
   using P = Published<unsigned long long>;
   using BS = cub::BlockScan<unsigned long long, ES_THREADS>;
   __shared__ typename BS::TempStorage tmp;
@@ -561,7 +559,6 @@ __global__ void __launch_bounds__(ES_THREADS) k_entry_scan(EntryScanArgs a, uint
       if (lane == 0) st_relaxed(state + t, (t == 0 ? P::PREFIX : P::AGGREGATE) | agg);
       uint32_t left = t;
       long long t0 = 0;
-      bool ok = true;
       while (left > 0) {
         const unsigned long long v = (uint32_t)lane < left ? ld_relaxed(state + (left - 1 - lane)) : P::PREFIX;
         const uint32_t ready = __ballot_sync(FULL, (v & ~P::VALUE) != 0);
@@ -575,32 +572,25 @@ __global__ void __launch_bounds__(ES_THREADS) k_entry_scan(EntryScanArgs a, uint
         if (take == 0) {
           const long long now = clock64();
           if (t0 == 0) t0 = now;
-          ok = !__any_sync(FULL, now - t0 > WAIT_CYCLES || ld_relaxed(hdr + SH_ABORT) != 0u);
-          if (!ok) break;
+          if (__any_sync(FULL, now - t0 >= wait)) {  // sum the next tile (a whole one) here
+            const uint64_t j0 = (uint64_t)(left - 1) * ES_TILE;
+            unsigned long long s = 0;
+            for (int k = lane; k < ES_TILE; k += 32) s += scan_in(a.in, a.perm, j0 + k);
+            before += warp_sum(s);
+            --left;
+            t0 = 0;
+          }
         } else {
           t0 = 0;
         }
       }
-      if (!ok) {
-        if (lane == 0) {
-          st_relaxed(hdr + SH_ABORT, 1u);
-          if (a.error_word != nullptr) atomicOr(a.error_word, ERR_TIMEOUT);
-          s_tile = 0xffffffffu;
-        }
-      } else if (lane == 0) {
+      if (lane == 0) {
         if (t > 0) st_relaxed(state + t, P::PREFIX | (before + agg));
         s_before = before;
         if (t + 1 == tiles) finish(before + agg);
       }
     }
     __syncthreads();
-    if (s_tile == 0xffffffffu) {  // gave up: no entries
-      if (tid == 0) {
-        if (a.total_u32 != nullptr) *a.total_u32 = 0u;
-        if (a.total_u64 != nullptr) *a.total_u64 = 0ull;
-      }
-      return;
-    }
     uint32_t r = (uint32_t)(s_before + excl);
     if (i0 + ES_ITEMS <= n) {
 #pragma unroll
@@ -884,7 +874,7 @@ int launch_sort_reset(const SortScratch& sc, cudaStream_t st) {
 
 int launch_entry_scan(const EntryScanArgs& a, const SortScratch& sc, int which, cudaStream_t st) {
   const int grid = grid_for(a.n_host, ES_TILE, 148 * 4);
-  k_entry_scan<<<grid, ES_THREADS, 0, st>>>(a, sc.scan_hdr[which], sc.scan_state[which]);
+  k_entry_scan<<<grid, ES_THREADS, 0, st>>>(a, sc.scan_hdr[which], sc.scan_state[which], sc.wait_cycles);
   return (int)cudaGetLastError();
 }
 

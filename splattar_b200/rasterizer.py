@@ -146,7 +146,7 @@ class Rasterizer:
 
     def set_wait_limits(self, copy_wait_cycles: int, drain_wait_cycles: int = 2_000_000_000):
         """Limits (SM cycles) of the fused projection backward + Adam kernel's bounded waits; a copy limit below
-        2e6 also bounds the sorts' waits, whose results do not depend on it."""
+        2e6 also bounds the waits of sorts and scans, whose results do not depend on it."""
         self._chk(lib().gs_rasterizer_set_wait_limits(self._h, copy_wait_cycles, drain_wait_cycles))
 
     def upload_scene(self, scene: SceneInput, stream: int = 0):

@@ -1,8 +1,9 @@
-"""A sort's block that runs out of its wait for an earlier tile counts that
-tile itself: with a wait limit of 0 (every look-back that meets an unpublished
-tile does so) the binning and the image are word for word those of the default
-limit. Sizes: a few look-back tiles up to more than the resident blocks, f32
-and deterministic values in the pairs, one view and several."""
+"""A sort's or entry scan's block that runs out of its wait for an earlier tile
+counts that tile itself: with a wait limit of 0 (every look-back that meets an
+unpublished tile does so) the binning and the image are word for word those of
+the default limit. Sizes: a few look-back tiles up to more than the resident
+blocks (296 of a sort pass, 592 of a scan), item and expansion indices in the
+pairs, one view and several."""
 import numpy as np
 import pytest
 
@@ -23,7 +24,8 @@ def _binning(r, cams, n, limit):
             r.read("out_color", 4 * pixels), total)
 
 
-@pytest.mark.parametrize("n,sizes", [(3000, [(200, 117)]), (9001, [(320, 240), (131, 90)]), (200000, [(1280, 720)] * 3)])
+@pytest.mark.parametrize("n,sizes", [(3000, [(200, 117)]), (9001, [(320, 240), (131, 90)]), (200000, [(1280, 720)] * 3),
+                                     (900000, [(160, 120)] * 3)])
 @pytest.mark.parametrize("deterministic", [False, True])
 def test_expired_waits_change_nothing(n, sizes, deterministic):
     cams = ring_cameras(sizes)
