@@ -147,10 +147,9 @@ __device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long 
 // memory latency per LB tiles. After `wait` cycles without the next tile's
 // word, `recount` (tile -> its own count) takes its place: the sum is the
 // same, and the loop ends whatever the other blocks do.
-template <typename W, class F>
+template <int LB, typename W, class F>
 __device__ __forceinline__ W look_back(const W* col, uint32_t stride, uint32_t t, long long wait, F&& recount) {
   using P = Published<W>;
-  constexpr int LB = 8;
   W sum = 0;
   uint32_t left = t;  // tiles [0, left) still to be summed
   long long t0 = 0;
@@ -201,10 +200,12 @@ __device__ __forceinline__ W look_back(const W* col, uint32_t stride, uint32_t t
 //
 // Against counting, scanning and scattering in five kernels per pass, each
 // pass reads its input once instead of twice, and a 32-bit sort takes 6
-// launches instead of 20. Whole 32-bit sorts, kernel time before and after:
-// 16 thousand pairs 69 -> 37 us, 300 thousand 76 -> 45, 1 million 97 -> 63,
-// 4 million 182 -> 169, 12 million 585 -> 470; 32 million pairs of 16 bits
-// 772 -> 614 us. A tile takes 6 us by itself (chains of ballots, barriers and
+// launches instead of 20. Whole 32-bit sorts of random keys in two arrays,
+// kernel time before and after: 16 thousand pairs 69 -> 37 us, 300 thousand
+// 76 -> 45, 1 million 97 -> 63, 4 million 182 -> 169, 12 million 585 -> 470; 32
+// million pairs of 16 bits 772 -> 614 us. Interleaved tile entries gain up to
+// 4 million (110 -> 87 us at 3.7 million) and lose beyond, also by chunks (below):
+// 8.6 million 164 -> 177 us, 33 million 545 -> 580. A tile takes 6 us by itself (chains of ballots, barriers and
 // L2 round trips), and the look-back grows with the tiles in flight: 2 blocks
 // of 512 threads per SM run the 4-million pass in 39 us, 3 blocks in 52, 6 of
 // 256 threads in 71, 8192-element tiles in 46 to 53; reading 16 or 32 tiles
@@ -231,12 +232,37 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d, int nbits, uint32_t 
   return peers;
 }
 
+// Many interleaved pairs go by chunks of whole tiles, one per half of a
+// resident block (chunk_pass). Against tiles by look-back, a tile's ranking
+// and writing then overlap the next tile's loads, and there is one look-back
+// per chunk; but every pass after the first reads its keys once more to count
+// them. Tile sorts (two passes) of entries in depth order, counting included:
+// 2.9 million 71 us by look-back and 78 by chunks, 4.3 million 97 and 100,
+// 5.8 million 129 and 123, 8.6 million 186 and 177, 18 million 391 and 336, 29
+// million 601 and 514, the 33 million of a 1080p frame 681 and 580. With one
+// pass (up to 256 tiles) look-back stays ahead (5.8 million 96 and 131), and
+// so it does for two arrays (32 million pairs of 16 bits: 294 us a pass by
+// look-back; 341 by chunks, counted and scanned by kernels of their own).
+constexpr int RC_THREADS = RS_THREADS / 2, RC_WARPS = RC_THREADS / 32;
+constexpr int RC_TILE = RS_TILE / 2, RC_ROUNDS = RC_TILE / RC_THREADS;
+constexpr uint32_t RC_CHUNKS = 148 * RS_CTAS * 2;
+constexpr int RC_GROUP = 25;  // chunks whose counts are summed first
+constexpr int RC_GROUPS = (RC_CHUNKS + RC_GROUP - 1) / RC_GROUP;
+constexpr uint64_t RC_MIN = 5000000;
+static_assert(RC_THREADS == RS_BINS, "one thread per digit");
+static_assert(RC_CHUNKS + RC_GROUPS <= RC_MIN / RS_TILE, "look-back words of the chunks and their groups");
+static_assert(RC_GROUPS <= RC_GROUP, "a look-back reads all groups at once");
+__device__ __forceinline__ uint64_t chunk_len(uint64_t n) {
+  return ((n + RC_CHUNKS - 1) / RC_CHUNKS + RC_TILE - 1) / RC_TILE * RC_TILE;
+}
+
 // Element access: two arrays, or one interleaved uint2 array.
 // SplitIO's optional gather (final pass only): gdst[position] = gsrc[value],
 // e.g. each item's tile count in sorted order for the entry scan, which then
 // reads it sequentially instead of through the permutation. PairIO's optional
 // value array (final pass only) receives the values alone.
 struct SplitIO {
+  static constexpr bool CHUNKS = false;
   const uint32_t* kin; const uint32_t* vin; uint32_t* kout; uint32_t* vout;
   const uint32_t* gsrc = nullptr; uint32_t* gdst = nullptr;
   SplitIO plain() const { SplitIO y = *this; y.gdst = nullptr; return y; }
@@ -250,6 +276,7 @@ struct SplitIO {
   }
 };
 struct PairIO {
+  static constexpr bool CHUNKS = true;
   const uint2* in; uint2* out;
   uint32_t* values = nullptr;
   PairIO plain() const { PairIO y = *this; y.values = nullptr; return y; }
@@ -269,6 +296,7 @@ struct PairIO {
 // sort, the ranges its final pass fills. Blocks take contiguous chunks of at
 // least 8 tiles' worth of threads, so that few elements flush few counters.
 constexpr int RH_THREADS = 512;
+static_assert(RC_MIN >= (uint64_t)RC_CHUNKS * 8 * RH_THREADS, "k_rs_hist has a block per chunk");
 template <class IO, typename W>
 __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, const uint32_t* n_dev, int passes,
                                                         int dbits, int key_bits, uint32_t* hdr, W* state,
@@ -280,9 +308,15 @@ __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, 
   const uint64_t gtid = (uint64_t)blockIdx.x * RH_THREADS + tid, gsize = (uint64_t)gridDim.x * RH_THREADS;
   for (uint64_t k = gtid; k < num_ranges; k += gsize) ranges[k] = make_uint2(0u, 0u);
   const uint64_t n = read_n(n_host, n_dev);
-  const uint64_t words = (n + RS_TILE - 1) / RS_TILE * RS_BINS;
-  for (uint64_t k = gtid; k < words; k += gsize) state[k] = 0;
-  const uint64_t chunk = max((n + gridDim.x - 1) / gridDim.x, (uint64_t)(8 * RH_THREADS));
+  const bool by_chunks = IO::CHUNKS && passes > 1 && n >= RC_MIN;
+  if (by_chunks) {  // (a chunk's own words are written below)
+    if (blockIdx.x < RC_GROUPS && tid < RS_BINS) state[(size_t)(RC_CHUNKS + blockIdx.x) * RS_BINS + tid] = 0;
+  } else {
+    const uint64_t words = (n + RS_TILE - 1) / RS_TILE * RS_BINS;
+    for (uint64_t k = gtid; k < words; k += gsize) state[k] = 0;
+  }
+  const uint64_t chunk =
+      by_chunks ? chunk_len(n) : max((n + gridDim.x - 1) / gridDim.x, (uint64_t)(8 * RH_THREADS));
   const uint64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   if (beg >= end) return;
   if (base != nullptr) io.skip(*base);
@@ -306,18 +340,162 @@ __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, 
   for (int k = tid; k < passes * RS_BINS; k += RH_THREADS) {
     const uint32_t c = (&s_h[0][0])[k];
     if (c) atomicAdd(hdr + SH_HIST + k, c);
+    if (by_chunks && k < RS_BINS)  // the first pass's counts of this chunk
+      state[(size_t)blockIdx.x * RS_BINS + k] = Published<W>::AGGREGATE | (W)c;
   }
 }
 
-// How many of a whole tile's keys have this digit (look_back's recount). Not
+// How many of a range's keys have this digit (look_back's recount). Not
 // inlined: it is hardly ever called, and the passes are short of registers
 // (sort of 4 million pairs 223 us without it, 220 with).
 template <class IO>
-__device__ __noinline__ uint32_t count_digit(IO io, uint64_t tile, int shift, uint32_t mask, uint32_t digit) {
+__device__ __noinline__ uint32_t count_digit(IO io, uint64_t beg, uint32_t len, int shift, uint32_t mask,
+                                             uint32_t digit) {
   uint32_t c = 0;
 #pragma unroll 8
-  for (int i = 0; i < RS_TILE; ++i) c += ((io.key(tile * RS_TILE + i) >> shift) & mask) == digit;
+  for (uint32_t i = 0; i < len; ++i) c += ((io.key(beg + i) >> shift) & mask) == digit;
   return c;
+}
+
+// A pass over many pairs (RC_MIN and more): half h of block b moves chunk
+// 2b + h of the input tile by tile, the next tile's elements in flight during
+// the write-out. It counts the chunk's digits first (the first pass finds them
+// in its look-back words, from k_rs_hist), adds the counts of the chunks before
+// it, its group's one by one and then the earlier groups', and needs no other
+// chunk after that. Only lower blocks and the own first half are waited for,
+// with look_back's bound. (Chunks by block number, not by ticket: 265 instead
+// of 282 us a pass at 33 million pairs.)
+template <class IO, typename W>
+__device__ __forceinline__ void chunk_pass(const IO& io, uint64_t n, int pass, int shift, int nbits, W* state,
+                                           W* next_state, uint2* ranges, uint32_t num_ranges, uint32_t b0,
+                                           long long wait, uint2* s_e, uint16_t (*s_wh)[RS_BINS], uint32_t* s_start,
+                                           uint32_t* s_gofs, uint32_t* s_warp, uint32_t digit_base) {
+  using P = Published<W>;
+  const int half = threadIdx.x / RC_THREADS, tid = threadIdx.x % RC_THREADS, lane = tid & 31, warp = tid >> 5;
+  auto sync_half = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(RC_THREADS) : "memory"); };
+  const uint32_t mask = (1u << nbits) - 1u;
+  const uint64_t len = chunk_len(n);
+  const uint32_t c = 2 * blockIdx.x + half, group = c / RC_GROUP, at = c % RC_GROUP;
+  const uint64_t beg = c * len, end = min(n, beg + len);
+  if (beg >= n) return;
+  W* mine = state + (size_t)c * RS_BINS + tid;
+  W* groups = state + (size_t)RC_CHUNKS * RS_BINS + tid;
+  if (next_state != nullptr) {
+    next_state[(size_t)c * RS_BINS + tid] = 0;
+    if (at == 0) next_state[(size_t)(RC_CHUNKS + group) * RS_BINS + tid] = 0;
+  }
+  W cnt;
+  if (pass == 0) {
+    cnt = *mine & P::VALUE;
+  } else {
+    uint32_t* h = reinterpret_cast<uint32_t*>(s_e);  // [RC_WARPS][RS_BINS]
+    for (int k = tid; k < RC_WARPS * RS_BINS; k += RC_THREADS) h[k] = 0;
+    sync_half();
+    uint32_t* hw = h + warp * RS_BINS;
+    uint64_t i = beg + tid;
+    for (; i + 3 * RC_THREADS < end; i += 4 * RC_THREADS) {
+      uint32_t k[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = io.key(i + u * RC_THREADS);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) atomicAdd(hw + ((k[u] >> shift) & mask), 1u);
+    }
+    for (; i < end; i += RC_THREADS) atomicAdd(hw + ((io.key(i) >> shift) & mask), 1u);
+    sync_half();
+    uint32_t s = 0;
+#pragma unroll
+    for (int w = 0; w < RC_WARPS; ++w) s += h[w * RS_BINS + tid];
+    cnt = s;
+    st_relaxed(mine, P::AGGREGATE | cnt);
+    sync_half();  // h is the staged tile's memory
+  }
+  auto recount = [&](uint64_t from, uint32_t chunks) {
+    return (W)count_digit(io, from * len, chunks * (uint32_t)len, shift, mask, (uint32_t)tid);
+  };
+  W before = 0;
+  if (at > 0)
+    before = look_back<RC_GROUP>(state + (size_t)(c - at) * RS_BINS + tid, RS_BINS, at, wait,
+                                 [&](uint32_t k) { return recount(c - at + k, 1); });
+  if (at == RC_GROUP - 1) st_relaxed(groups + (size_t)group * RS_BINS, P::AGGREGATE | (before + cnt));
+  if (group > 0)
+    before += look_back<RC_GROUP>(groups, RS_BINS, group, wait,
+                                  [&](uint32_t k) { return recount((uint64_t)k * RC_GROUP, RC_GROUP); });
+  uint32_t run = digit_base + (uint32_t)before;  // where this digit's next element goes
+  uint2 e[RC_ROUNDS];
+  auto load_tile = [&](uint64_t t0) {
+    const int tn = (int)min((uint64_t)RC_TILE, end - t0);
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const int idx = warp * (RC_ROUNDS * 32) + r * 32 + lane;
+      e[r] = idx < tn ? io.load(t0 + idx) : make_uint2(0u, 0u);
+    }
+  };
+  load_tile(beg);
+  for (uint64_t t0 = beg; t0 < end; t0 += RC_TILE) {
+    const int tn = (int)min((uint64_t)RC_TILE, end - t0);
+    for (int k = tid; k < RC_WARPS * RS_BINS / 2; k += RC_THREADS) reinterpret_cast<uint32_t*>(&s_wh[0][0])[k] = 0;
+    sync_half();
+    uint32_t pre[RC_ROUNDS];  // ranks within (warp, digit)
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const int idx = warp * (RC_ROUNDS * 32) + r * 32 + lane;
+      const bool valid = idx < tn;
+      const uint32_t d = (e[r].x >> shift) & mask;
+      const uint32_t act = __ballot_sync(FULL, valid);
+      const uint32_t peers = match_digit(d, nbits, act);
+      uint32_t basev = 0;
+      if (valid) basev = s_wh[warp][d];
+      __syncwarp();
+      if (valid && (peers & lanemask_lt()) == 0) s_wh[warp][d] = (uint16_t)(basev + __popc(peers));
+      __syncwarp();
+      pre[r] = basev + __popc(peers & lanemask_lt());
+    }
+    sync_half();
+    uint32_t s = 0;
+#pragma unroll
+    for (int w = 0; w < RC_WARPS; ++w) {
+      const uint32_t x = s_wh[w][tid];
+      s_wh[w][tid] = (uint16_t)s;
+      s += x;
+    }
+    uint32_t excl = s;  // inclusive over the warp, then exclusive over the half
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(FULL, excl, o);
+      if (lane >= o) excl += x;
+    }
+    if (lane == 31) s_warp[warp] = excl;
+    sync_half();
+    excl -= s;
+#pragma unroll
+    for (int w = 0; w < RC_WARPS; ++w)
+      if (w < warp) excl += s_warp[w];
+    s_start[tid] = excl;
+    s_gofs[tid] = run - excl;  // output position = s_gofs[d] + position in the tile
+    run += s;
+    sync_half();
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const int idx = warp * (RC_ROUNDS * 32) + r * 32 + lane;
+      if (idx < tn) {
+        const uint32_t d = (e[r].x >> shift) & mask;
+        s_e[s_start[d] + s_wh[warp][d] + pre[r]] = e[r];
+      }
+    }
+    if (t0 + RC_TILE < end) load_tile(t0 + RC_TILE);
+    sync_half();
+#pragma unroll 4
+    for (int i = tid; i < tn; i += RC_THREADS) {
+      const uint2 v = s_e[i];
+      const uint32_t pos = s_gofs[(v.x >> shift) & mask] + (uint32_t)i;
+      io.store((size_t)pos, v);
+      if (ranges != nullptr && v.x < num_ranges) {
+        if (i == 0 || s_e[i - 1].x != v.x) atomicMax(&ranges[v.x].x, ~(b0 + pos));
+        if (i == tn - 1 || s_e[i + 1].x != v.x) atomicMax(&ranges[v.x].y, b0 + pos + 1u);
+      }
+    }
+    sync_half();
+  }
 }
 
 // ranges (final pass of a key sort only, else null): every run of one key
@@ -329,14 +507,15 @@ __device__ __noinline__ uint32_t count_digit(IO io, uint64_t tile, int shift, ui
 // the lower digits the earlier passes sorted.
 template <class IO, typename W>
 __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t n_host, const uint32_t* n_dev,
-                                                                 int pass, int shift, int nbits, uint32_t* hdr,
-                                                                 W* state, W* next_state, uint2* ranges,
+                                                                 int pass, int passes, int shift, int nbits,
+                                                                 uint32_t* hdr, W* state, W* next_state, uint2* ranges,
                                                                  uint32_t num_ranges, const unsigned long long* base,
                                                                  long long wait) {
   using P = Published<W>;
   __shared__ uint2 s_e[RS_TILE];
   __shared__ uint16_t s_wh[RS_WARPS][RS_BINS];
-  __shared__ uint32_t s_start[RS_BINS], s_gofs[RS_BINS];
+  constexpr int HALVES = IO::CHUNKS ? 2 : 1;  // chunk_pass: each half has its own
+  __shared__ uint32_t s_start[HALVES * RS_BINS], s_gofs[HALVES * RS_BINS];
   __shared__ uint32_t s_tile;
   using BS = cub::BlockScan<uint32_t, RS_THREADS>;
   __shared__ typename BS::TempStorage tmp;
@@ -349,6 +528,19 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
   const uint32_t mask = (1u << nbits) - 1u;
   uint32_t digit_base;
   BS(tmp).ExclusiveSum(tid < RS_BINS ? hdr[SH_HIST + pass * RS_BINS + tid] : 0u, digit_base);
+  if constexpr (IO::CHUNKS) {
+    if (passes > 1 && n >= RC_MIN) {
+      __shared__ uint32_t s_warp[2][RC_WARPS];
+      if (tid < RS_BINS) s_start[tid] = s_start[RS_BINS + tid] = digit_base;
+      __syncthreads();
+      digit_base = s_start[tid];
+      const int half = tid / RC_THREADS;
+      chunk_pass<IO, W>(io, n, pass, shift, nbits, state, next_state, ranges, num_ranges, b0, wait,
+                        s_e + half * RC_TILE, s_wh + half * RC_WARPS, s_start + half * RS_BINS,
+                        s_gofs + half * RS_BINS, s_warp[half], digit_base);
+      return;
+    }
+  }
   for (;;) {
     if (tid == 0) s_tile = atomicAdd(hdr + SH_TICKET + pass, 1u);
     for (int k = tid; k < RS_WARPS * RS_BINS / 2; k += RS_THREADS) reinterpret_cast<uint32_t*>(&s_wh[0][0])[k] = 0;
@@ -407,8 +599,8 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
     }
     W before = 0;
     if (t > 0 && tid <= (int)mask) {
-      before = look_back(state + tid, RS_BINS, t, wait, [&](uint32_t tile) {
-        return (W)count_digit(io, tile, shift, mask, (uint32_t)tid);
+      before = look_back<8>(state + tid, RS_BINS, t, wait, [&](uint32_t tile) {
+        return (W)count_digit(io, (uint64_t)tile * RS_TILE, RS_TILE, shift, mask, (uint32_t)tid);
       });
       st_relaxed(mine, P::PREFIX | (before + (W)cnt));
     }
@@ -893,7 +1085,7 @@ int radix_passes(IO io, uint64_t n_host, const uint32_t* n_dev, int key_bits, co
   for (int p = 0; p < passes; ++p) {
     const int shift = p * dbits, nbits = std::min(dbits, key_bits - shift);
     const bool last = p + 1 == passes;
-    k_rs_pass<IO, W><<<grid, RS_THREADS, 0, st>>>(last ? io : io.plain(), n_host, n_dev, p, shift, nbits, h,
+    k_rs_pass<IO, W><<<grid, RS_THREADS, 0, st>>>(last ? io : io.plain(), n_host, n_dev, p, passes, shift, nbits, h,
                                                   state[p & 1], last ? nullptr : state[(p + 1) & 1],
                                                   last ? ranges : nullptr, num_ranges, base, sc.wait_cycles);
     swap(io);
