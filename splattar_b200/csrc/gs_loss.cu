@@ -363,31 +363,74 @@ constexpr int BM_THREADS = 384;                  // 3 channels × 4 row segments
 constexpr size_t BM_SMEM = sizeof(float2) * (3 * EXT32 * BIG_PITCH + 6 * EXT32 * BIG_ROW);
 // Two packed maps per channel: (μx, μy) and (E[x² + y²], E[xy]); SSIM needs
 // the two variances as a sum only, so four maps do where five were blurred.
-// x and y are shifted by −0.5 (outside the image too), which leaves variances
-// and covariances as they are and shrinks the squares that cancel in them.
-// A vertical item slides both maps of its channel down 8 rows and forms that
+// x and y are shifted by one value per tile and channel (tile_shift; outside
+// the image too), which leaves variances and covariances as they are and shrinks
+// the squares that cancel in them; L1 is summed from the unshifted values. A
+// vertical item slides both maps of its channel down 8 rows and forms that
 // channel's coefficients from registers.
-constexpr float SHIFT = 0.5f;
+constexpr int BM_LOADS = (EXT32 * EXT32 + BM_THREADS - 1) / BM_THREADS;  // staged pixels per thread
+
+// Mean of 8 × 4 sampled pixels of the tile, dark pixels and those like their
+// diagonal neighbour counting most: SSIM is most sensitive to rounding where
+// the variance is small beside C2, and a dark flat background must not be
+// shifted by a bright or busy object in the same tile. The gradient's relative
+// error against 64 bits, 16-pixel tiles unshifted, here, and with a fixed 0.5:
+// smooth mid-tones 6.9e-6, 1.6e-6, 2.5e-6; values up to 0.05 2.4e-7, 2.4e-7,
+// 7.3e-6; objects on black 2.8e-7, 3.2e-7, 2.9e-6 (1.7e-6 with the plain mean).
+// Called by whole warps.
+__device__ __forceinline__ float tile_shift(const SsimArgs& a, const TileLoc& L, int lane, int ch) {
+  const int x0 = min(L.x0 + 2 + 4 * (lane & 7), L.W - 1), y0 = min(L.y0 + 4 + 8 * (lane >> 3), L.H - 1);
+  const int x1 = min(x0 + 1, L.W - 1), y1 = min(y0 + 1, L.H - 1);
+  const long long p = 4 * (L.pix_base + (long long)y0 * L.W + x0) + ch;
+  const long long q = 4 * (L.pix_base + (long long)y1 * L.W + x1) + ch;
+  const float* img = &a.img->x;
+  const float* target = &a.target->x;
+  const float x = img[p], y = target[p], dx = x - img[q], dy = y - target[q], m = 0.5f * (x + y);
+  const float w = __fdividef(1.0f, (9e-4f + dx * dx + dy * dy) * (0.1f + m * m));
+  const float s = __fdividef(warp_sum(w * m), warp_sum(w));
+  return fabsf(s) < 1e15f ? s : 0.f;  // (no shift beside NaN and infinities)
+}
 __global__ void __launch_bounds__(BM_THREADS, 2) k_ssim_moments_big(SsimArgs a) {
   extern __shared__ __align__(16) unsigned char big_smem[];
   float2* s_in = reinterpret_cast<float2*>(big_smem);       // [ch][EXT32][BIG_PITCH]
   float2* s_h = s_in + 3 * EXT32 * BIG_PITCH;               // [ch·2 + map][EXT32][BIG_ROW]
   __shared__ double s_red[2][BM_THREADS / 32];
+  __shared__ float s_shift[3];
   const int tid = threadIdx.x;
   const TileLoc L = locate<T32>(a, blockIdx.x);
-  for (int k = tid; k < EXT32 * EXT32; k += BM_THREADS) {
-    const int ly = k / EXT32, lx = k - ly * EXT32;
-    const int gx = L.x0 + lx - HALO, gy = L.y0 + ly - HALO;
-    float4 xv = make_float4(0, 0, 0, 0), yv = xv;
-    if (gx >= 0 && gy >= 0 && gx < L.W && gy < L.H) {
-      const long long p = L.pix_base + (long long)gy * L.W + gx;
-      xv = a.img[p];
-      yv = a.target[p];
+  float l1 = 0.f, ss = 0.f, shift[3];
+  if (tid < 3 * 32) {
+    const float s = tile_shift(a, L, tid & 31, tid >> 5);
+    if ((tid & 31) == 0) s_shift[tid >> 5] = s;
+  }
+  {
+    float4 xv[BM_LOADS], yv[BM_LOADS];  // all in flight beside the samples
+#pragma unroll
+    for (int u = 0; u < BM_LOADS; ++u) {
+      const int k = tid + u * BM_THREADS, ly = k / EXT32, lx = k - ly * EXT32;
+      const int gx = L.x0 + lx - HALO, gy = L.y0 + ly - HALO;
+      xv[u] = yv[u] = make_float4(0, 0, 0, 0);
+      if (k < EXT32 * EXT32 && gx >= 0 && gy >= 0 && gx < L.W && gy < L.H) {
+        const long long p = L.pix_base + (long long)gy * L.W + gx;
+        xv[u] = a.img[p];
+        yv[u] = a.target[p];
+      }
     }
-    float2* d = s_in + ly * BIG_PITCH + lx;
-    d[0] = make_float2(xv.x - SHIFT, yv.x - SHIFT);
-    d[EXT32 * BIG_PITCH] = make_float2(xv.y - SHIFT, yv.y - SHIFT);
-    d[2 * EXT32 * BIG_PITCH] = make_float2(xv.z - SHIFT, yv.z - SHIFT);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) shift[k] = s_shift[k];
+#pragma unroll
+    for (int u = 0; u < BM_LOADS; ++u) {
+      const int k = tid + u * BM_THREADS, ly = k / EXT32, lx = k - ly * EXT32;
+      if (k >= EXT32 * EXT32) break;
+      const float4 x = xv[u], y = yv[u];
+      if ((unsigned)(lx - HALO) < T32 && (unsigned)(ly - HALO) < T32)  // (outside the image both are zero)
+        l1 += fabsf(x.x - y.x) + fabsf(x.y - y.y) + fabsf(x.z - y.z);
+      float2* d = s_in + ly * BIG_PITCH + lx;
+      d[0] = make_float2(x.x - shift[0], y.x - shift[0]);
+      d[EXT32 * BIG_PITCH] = make_float2(x.y - shift[1], y.y - shift[1]);
+      d[2 * EXT32 * BIG_PITCH] = make_float2(x.z - shift[2], y.z - shift[2]);
+    }
   }
   float w[6];
 #pragma unroll
@@ -406,16 +449,14 @@ __global__ void __launch_bounds__(BM_THREADS, 2) k_ssim_moments_big(SsimArgs a) 
   }
   __syncthreads();
   // Vertical: item = (channel, 8-row segment, column).
-  float l1 = 0.f, ss = 0.f;
   {
     const int c = tid & 31, sg = (tid >> 5) & 3, ch = tid >> 7;
     const int gx = L.x0 + c;
     const float2* M = s_h + (ch * 2 * EXT32 + 8 * sg) * BIG_ROW + c;
     const float2* S = M + EXT32 * BIG_ROW;
-    const float2* X = s_in + (ch * EXT32 + 8 * sg + HALO) * BIG_PITCH + c + HALO;
     const float inv_n3 = 1.0f / (3.0f * (float)L.W * (float)L.H);
     const float C1 = 1e-4f, C2 = 9e-4f;
-    const float dw = -a.w_ssim * inv_n3;
+    const float dw = -a.w_ssim * inv_n3, up = ch == 0 ? shift[0] : ch == 1 ? shift[1] : shift[2];
     // this channel's places: r and g are the halves of planes 0..2, b has
     // plane 3 (Cμ, Cx²) and the scalar plane (Cxy)
     const size_t st2 = 2 * a.coef_stride;
@@ -439,10 +480,8 @@ __global__ void __launch_bounds__(BM_THREADS, 2) k_ssim_moments_big(SsimArgs a) 
       for (int i = 0; i < TAPS - 1; ++i) { wm[i] = wm[i + 1]; ws[i] = ws[i + 1]; }
       const int gy = L.y0 + 8 * sg + o;
       if (gx < L.W && gy < L.H) {
-        const float2 xy = X[o * BIG_PITCH];
-        l1 += fabsf(xy.x - xy.y);
         const float s2 = b.x - mu.x * mu.x - mu.y * mu.y, sxy = b.y - mu.x * mu.y;
-        const float mu_x = mu.x + SHIFT, mu_y = mu.y + SHIFT;
+        const float mu_x = mu.x + up, mu_y = mu.y + up;
         const float p = mu_x * mu_x + mu_y * mu_y + C1;
         const float qd = s2 + C2;
         const float ip = __fdividef(1.0f, p), iq = __fdividef(1.0f, qd);  // as in k_ssim_moments
@@ -601,9 +640,11 @@ int launch_ssim(const SsimArgs& a_in, cudaStream_t st) {
   s = g[0];
   for (int k = 1; k <= 5; ++k) s += 2 * g[k];
   for (int k = 0; k <= 5; ++k) a.w[k] = (float)(g[k] / s);
-  // Moments on 32×32 tiles from five per SM on: 720p (920 tiles) 38.0 -> 34.5
-  // us, 1080p 80.0 -> 72.6, 4K 300 -> 270; at 640x480 (300 tiles) they took
-  // 16.1 us against 15.1, at 800x600 (475) 20.8 both ways. (The gradient
+  // Moments on 32×32 tiles from five per SM on: 720p (920 tiles) 38.4 -> 36.7
+  // us, 1080p 80.2 -> 75.2, 4K 300 -> 284 (of which the shift costs 1, 3 and 17
+  // us; with its samples loaded beside the staged pixels instead of before them
+  // 38.0, 79, 300); at 640x480 (300 tiles) they took 16.1 us against 15.1, at
+  // 800x600 (475) 20.8 both ways. (The gradient
   // kernel gained nothing from them: 1080p 80.6 against 81.3 us, 4K 299 against
   // 293.)
   if (a.total_tiles32 >= 5 * 148) {
