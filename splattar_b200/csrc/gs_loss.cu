@@ -644,10 +644,12 @@ int launch_ssim(const SsimArgs& a_in, cudaStream_t st) {
   // us, 1080p 80.2 -> 75.2, 4K 300 -> 284 (of which the shift costs 1, 3 and 17
   // us; with its samples loaded beside the staged pixels instead of before them
   // 38.0, 79, 300); at 640x480 (300 tiles) they took 16.1 us against 15.1, at
-  // 800x600 (475) 20.8 both ways. (The gradient
+  // 800x600 (475) 20.8 both ways. Only where they replace at least 3.5 small
+  // tiles each: 33 pixels wide (3.0, 752 tiles) they took 28.4 us against 24.0,
+  // 100 wide (3.5, 1000 tiles) 36.3 against 36.1. (The gradient
   // kernel gained nothing from them: 1080p 80.6 against 81.3 us, 4K 299 against
   // 293.)
-  if (a.total_tiles32 >= 5 * 148) {
+  if (a.total_tiles32 >= 5 * 148 && 2 * a.total_tiles16 >= 7 * a.total_tiles32) {
     const cudaError_t e =
         cudaFuncSetAttribute(k_ssim_moments_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BM_SMEM);
     if (e != cudaSuccess) return (int)e;

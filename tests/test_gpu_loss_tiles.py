@@ -1,5 +1,6 @@
 """The losses' block and tile edges: L1+SSIM on images of many 32-pixel tiles
-(whole, and a pixel more or less each way) and the normal loss summed over
+(whole, and a pixel more or less each way; narrow ones, which go by 16-pixel
+tiles when too little of the large ones is image) and the normal loss summed over
 several blocks of several views, against the oracle."""
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ from splattar_b200 import Rasterizer
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("W,H", [(1024, 768), (1023, 801), (33, 12001), (12001, 33)])
+@pytest.mark.parametrize("W,H", [(1024, 768), (1023, 801), (33, 12001), (12001, 33), (125, 8001), (8001, 125)])
 @pytest.mark.parametrize("level", [(0.0, 1.0), (0.0, 0.05), (0.9, 1.6)])
 def test_l1_ssim_large_tiles(W, H, level):
     """Bounds of test_l1_ssim_matches_oracle."""
