@@ -448,10 +448,13 @@ gs_status gs_binner_buffer(gs_binner* b, uint32_t which, void** dptr, size_t* by
 /* ---- RadixSorter / PrefixSum (crates/gs-wgpu/src/{sort,prefix_sum}.rs) ----
  * Stable LSD sort of n (key, value) u32 pairs on bits [0, key_bits), in
  * place; and an exclusive u32 scan with the total written to *total_dev.
- * Both take caller device pointers. The scan's scratch is allocated on first
- * use; the sort takes its own from a memory pool of the library in stream
- * order, which keeps up to 512 MiB between calls (both held until
- * gs_shutdown). */
+ * Both take caller device pointers, and their scratch in stream order from a
+ * memory pool of the library (one per device), which keeps up to 512 MiB
+ * between calls; gs_shutdown, after which both work as on first use, gives it
+ * back. Calls on several streams and threads may overlap. The sort
+ * synchronises its stream; the scan does not and can be captured after a first
+ * call on the device (scans in graphs share one array, so replays that overlap
+ * race). */
 gs_status gs_radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, uint32_t key_bits, void* stream);
 gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev, void* stream);
 

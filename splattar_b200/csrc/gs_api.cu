@@ -1942,48 +1942,64 @@ extern "C" gs_status gs_binner_buffer(gs_binner* b, uint32_t which, void** dptr,
 
 // ------------------------------------------------------- sort / scan API
 namespace {
-// Scratch of the public scan, and the memory pool of the public sort, on the
-// device of the last call. The pool serves buffers in stream order, so calls
-// on several streams and threads have their own; it keeps up to
-// SORT_POOL_KEEP bytes between calls (the default pool keeps none past a
-// synchronisation, and mapping 32 MB afresh took 0.45 of 0.71 ms of a
-// 4M-pair sort) and is given back by gs_shutdown.
-constexpr uint64_t SORT_POOL_KEEP = 512ull << 20;
+// Memory pools of the public sort and scan, one per device they ran on. A pool
+// serves buffers in stream order, so calls on several streams and threads have
+// their own; it keeps up to POOL_KEEP bytes between calls (the default pool
+// keeps none past a synchronisation, and mapping 32 MB afresh took 0.45 of 0.71
+// ms of a 4M-pair sort). `captured` holds the block sums of scans recorded
+// into graphs, which cannot take theirs from the pool (a graph that allocates
+// can neither be updated nor be instantiated twice). gs_shutdown gives all of
+// it back.
+constexpr uint64_t POOL_KEEP = 512ull << 20;
+constexpr int MAX_DEVICES = 64;
+struct DeviceScratch {
+  cudaMemPool_t pool = nullptr;
+  void* captured = nullptr;
+};
 struct GlobalScratch {
   std::mutex mu;
-  int device = -1;
-  void* scan = nullptr;
-  cudaMemPool_t pool = nullptr;
-  void release() {
-    if (scan) cudaFree(scan);
-    if (pool) cudaMemPoolDestroy(pool);
-    scan = nullptr;
-    pool = nullptr;
-    device = -1;
-  }
+  DeviceScratch dev[MAX_DEVICES];
 };
 GlobalScratch g_scratch;
 
-// Makes the scratch exist on the current device (under the lock).
-gs_status global_scratch_locked() {
+// The current device's scratch, made on first use (under the lock).
+gs_status global_scratch_locked(DeviceScratch** out) {
   int dev = 0;
-  cudaGetDevice(&dev);
-  if (g_scratch.device != dev) {
-    g_scratch.release();
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev >= MAX_DEVICES) return fail(nullptr, GS_ERR_CAPACITY, "scratch: more than 64 devices");
+  if (e != cudaSuccess) return fail(nullptr, GS_ERR_CUDA, std::string("scratch: ") + cudaGetErrorString(e));
+  DeviceScratch& d = g_scratch.dev[dev];
+  if (!d.pool) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    uint64_t keep = SORT_POOL_KEEP;
-    cudaError_t e = cudaMalloc(&g_scratch.scan, scan_scratch_bytes());
-    if (e == cudaSuccess) e = cudaMemPoolCreate(&g_scratch.pool, &props);
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(g_scratch.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    uint64_t keep = POOL_KEEP;
+    void* scan = nullptr;
+    cudaMemPool_t pool = nullptr;
+    e = cudaMalloc(&scan, scan_scratch_bytes());
+    if (e == cudaSuccess) e = cudaMemPoolCreate(&pool, &props);
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) {
-      g_scratch.release();
+      if (scan) cudaFree(scan);
+      if (pool) cudaMemPoolDestroy(pool);
       return fail(nullptr, GS_ERR_CUDA, std::string("scratch: ") + cudaGetErrorString(e));
     }
-    g_scratch.device = dev;
+    d.captured = scan;
+    d.pool = pool;
   }
+  *out = &d;
+  return GS_OK;
+}
+
+// A buffer of the current device's pool, in stream order.
+gs_status pool_alloc(void** out, size_t bytes, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_scratch.mu);
+  DeviceScratch* d = nullptr;
+  const gs_status s = global_scratch_locked(&d);
+  if (s) return s;
+  const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, d->pool, st);
+  if (e != cudaSuccess) return fail(nullptr, GS_ERR_CUDA, std::string("scratch: ") + cudaGetErrorString(e));
   return GS_OK;
 }
 }  // namespace
@@ -1996,14 +2012,8 @@ extern "C" gs_status gs_radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_
   // One buffer: the other half of the ping-pong, then the pass scratch.
   const size_t arr = (size_t)((n * 4 + 255) / 256 * 256);
   unsigned char* buf = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_scratch.mu);
-    gs_status s = global_scratch_locked();
-    if (s) return s;
-    const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&buf), 2 * arr + sort_scratch_bytes(n, 0),
-                                                  g_scratch.pool, st);
-    if (e != cudaSuccess) return fail(nullptr, GS_ERR_CUDA, std::string("sort buffers: ") + cudaGetErrorString(e));
-  }
+  const gs_status ps = pool_alloc(reinterpret_cast<void**>(&buf), 2 * arr + sort_scratch_bytes(n, 0), st);
+  if (ps) return ps;
   uint32_t* k1 = reinterpret_cast<uint32_t*>(buf);
   uint32_t* v1 = reinterpret_cast<uint32_t*>(buf + arr);
   const SortScratch sc = sort_scratch(buf + 2 * arr, n, 0);
@@ -2025,20 +2035,34 @@ extern "C" gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, ui
                                            void* stream) {
   if ((!in || !out) && n) return fail(nullptr, GS_ERR_INVALID_ARG, "bad scan args");
   if (n >= 0xffffffffull) return fail(nullptr, GS_ERR_INVALID_ARG, "scan length must be < 2^32");
+  cudaStream_t st = S(stream);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const cudaError_t ce = cudaStreamIsCapturing(st, &cap);
+  if (ce != cudaSuccess) return fail(nullptr, GS_ERR_CUDA, std::string("scan: ") + cudaGetErrorString(ce));
+  const bool captured = cap != cudaStreamCaptureStatusNone;
   void* scan = nullptr;
-  {
+  if (captured) {
     std::lock_guard<std::mutex> lk(g_scratch.mu);
-    gs_status s = global_scratch_locked();
+    DeviceScratch* d = nullptr;
+    const gs_status s = global_scratch_locked(&d);
     if (s) return s;
-    scan = g_scratch.scan;
+    scan = d->captured;
+  } else {
+    const gs_status s = pool_alloc(&scan, scan_scratch_bytes(), st);
+    if (s) return s;
   }
-  int e = launch_scan(in, nullptr, out, n, nullptr, total_dev, nullptr, scan, S(stream));
+  int e = launch_scan(in, nullptr, out, n, nullptr, total_dev, nullptr, scan, st);
+  if (!captured) cudaFreeAsync(scan, st);
   if (e) return fail(nullptr, GS_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
   return GS_OK;
 }
 
 extern "C" gs_status gs_shutdown(void) {
   std::lock_guard<std::mutex> lk(g_scratch.mu);
-  g_scratch.release();
+  for (DeviceScratch& d : g_scratch.dev) {
+    if (d.captured) cudaFree(d.captured);
+    if (d.pool) cudaMemPoolDestroy(d.pool);
+    d = DeviceScratch{};
+  }
   return GS_OK;
 }
