@@ -205,7 +205,7 @@ __device__ __forceinline__ W look_back(const W* col, uint32_t stride, uint32_t t
 // 76 -> 45, 1 million 97 -> 63, 4 million 182 -> 169, 12 million 585 -> 470; 32
 // million pairs of 16 bits 772 -> 614 us. Interleaved tile entries gain up to
 // 4 million (110 -> 87 us at 3.7 million) and lose beyond, also by chunks (below):
-// 8.6 million 164 -> 177 us, 33 million 545 -> 580. A tile takes 6 us by itself (chains of ballots, barriers and
+// 8.6 million 164 -> 175 us, 33 million 545 -> 570. A tile takes 6 us by itself (chains of ballots, barriers and
 // L2 round trips), and the look-back grows with the tiles in flight: 2 blocks
 // of 512 threads per SM run the 4-million pass in 39 us, 3 blocks in 52, 6 of
 // 256 threads in 71, 8192-element tiles in 46 to 53; reading 16 or 32 tiles
@@ -238,8 +238,8 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d, int nbits, uint32_t 
 // per chunk; but every pass after the first reads its keys once more to count
 // them. Tile sorts (two passes) of entries in depth order, counting included:
 // 2.9 million 71 us by look-back and 78 by chunks, 4.3 million 97 and 100,
-// 5.8 million 129 and 123, 8.6 million 186 and 177, 18 million 391 and 336, 29
-// million 601 and 514, the 33 million of a 1080p frame 681 and 580. With one
+// 5.8 million 129 and 123, 8.6 million 186 and 175, 18 million 391 and 336, 29
+// million 601 and 514, the 33 million of a 1080p frame 681 and 570. With one
 // pass (up to 256 tiles) look-back stays ahead (5.8 million 96 and 131), and
 // so it does for two arrays (32 million pairs of 16 bits: 294 us a pass by
 // look-back; 341 by chunks, counted and scanned by kernels of their own).
@@ -275,8 +275,9 @@ struct SplitIO {
     if (gdst != nullptr) gdst[g] = __ldg(gsrc + e.y);
   }
 };
+template <bool BY_CHUNKS>  // RC_MIN elements and more go by chunks
 struct PairIO {
-  static constexpr bool CHUNKS = true;
+  static constexpr bool CHUNKS = BY_CHUNKS;
   const uint2* in; uint2* out;
   uint32_t* values = nullptr;
   PairIO plain() const { PairIO y = *this; y.values = nullptr; return y; }
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, 
   const uint64_t gtid = (uint64_t)blockIdx.x * RH_THREADS + tid, gsize = (uint64_t)gridDim.x * RH_THREADS;
   for (uint64_t k = gtid; k < num_ranges; k += gsize) ranges[k] = make_uint2(0u, 0u);
   const uint64_t n = read_n(n_host, n_dev);
-  const bool by_chunks = IO::CHUNKS && passes > 1 && n >= RC_MIN;
+  const bool by_chunks = IO::CHUNKS && n >= RC_MIN;
   if (by_chunks) {  // (a chunk's own words are written below)
     if (blockIdx.x < RC_GROUPS && tid < RS_BINS) state[(size_t)(RC_CHUNKS + blockIdx.x) * RS_BINS + tid] = 0;
   } else {
@@ -345,15 +346,22 @@ __global__ void __launch_bounds__(RH_THREADS) k_rs_hist(IO io, uint64_t n_host, 
   }
 }
 
-// How many of a range's keys have this digit (look_back's recount). Not
-// inlined: it is hardly ever called, and the passes are short of registers
-// (sort of 4 million pairs 223 us without it, 220 with).
+// How many of a whole tile's, or a range of tiles', keys have this digit
+// (look_back's recount). Not inlined: it is hardly ever called, and the passes
+// are short of registers (sort of 4 million pairs 223 us without it, 220 with).
 template <class IO>
-__device__ __noinline__ uint32_t count_digit(IO io, uint64_t beg, uint32_t len, int shift, uint32_t mask,
-                                             uint32_t digit) {
+__device__ __noinline__ uint32_t count_digit(IO io, uint64_t tile, int shift, uint32_t mask, uint32_t digit) {
   uint32_t c = 0;
 #pragma unroll 8
-  for (uint32_t i = 0; i < len; ++i) c += ((io.key(beg + i) >> shift) & mask) == digit;
+  for (int i = 0; i < RS_TILE; ++i) c += ((io.key(tile * RS_TILE + i) >> shift) & mask) == digit;
+  return c;
+}
+template <class IO>
+__device__ __noinline__ uint32_t count_range(IO io, uint64_t beg, uint64_t end, int shift, uint32_t mask,
+                                             uint32_t digit) {
+  uint32_t c = 0;
+#pragma unroll 4
+  for (uint64_t i = beg; i < end; ++i) c += ((io.key(i) >> shift) & mask) == digit;
   return c;
 }
 
@@ -372,7 +380,10 @@ __device__ __forceinline__ void chunk_pass(const IO& io, uint64_t n, int pass, i
                                            uint32_t* s_gofs, uint32_t* s_warp, uint32_t digit_base) {
   using P = Published<W>;
   const int half = threadIdx.x / RC_THREADS, tid = threadIdx.x % RC_THREADS, lane = tid & 31, warp = tid >> 5;
-  auto sync_half = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(RC_THREADS) : "memory"); };
+  auto sync_half = [&] {
+    if (half) asm volatile("bar.sync 2, %0;" ::"n"(RC_THREADS) : "memory");
+    else asm volatile("bar.sync 1, %0;" ::"n"(RC_THREADS) : "memory");
+  };
   const uint32_t mask = (1u << nbits) - 1u;
   const uint64_t len = chunk_len(n);
   const uint32_t c = 2 * blockIdx.x + half, group = c / RC_GROUP, at = c % RC_GROUP;
@@ -410,7 +421,7 @@ __device__ __forceinline__ void chunk_pass(const IO& io, uint64_t n, int pass, i
     sync_half();  // h is the staged tile's memory
   }
   auto recount = [&](uint64_t from, uint32_t chunks) {
-    return (W)count_digit(io, from * len, chunks * (uint32_t)len, shift, mask, (uint32_t)tid);
+    return (W)count_range(io, from * len, (from + chunks) * len, shift, mask, (uint32_t)tid);
   };
   W before = 0;
   if (at > 0)
@@ -507,7 +518,7 @@ __device__ __forceinline__ void chunk_pass(const IO& io, uint64_t n, int pass, i
 // the lower digits the earlier passes sorted.
 template <class IO, typename W>
 __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t n_host, const uint32_t* n_dev,
-                                                                 int pass, int passes, int shift, int nbits,
+                                                                 int pass, int shift, int nbits,
                                                                  uint32_t* hdr, W* state, W* next_state, uint2* ranges,
                                                                  uint32_t num_ranges, const unsigned long long* base,
                                                                  long long wait) {
@@ -529,7 +540,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
   uint32_t digit_base;
   BS(tmp).ExclusiveSum(tid < RS_BINS ? hdr[SH_HIST + pass * RS_BINS + tid] : 0u, digit_base);
   if constexpr (IO::CHUNKS) {
-    if (passes > 1 && n >= RC_MIN) {
+    if (n >= RC_MIN) {
       __shared__ uint32_t s_warp[2][RC_WARPS];
       if (tid < RS_BINS) s_start[tid] = s_start[RS_BINS + tid] = digit_base;
       __syncthreads();
@@ -600,7 +611,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
     W before = 0;
     if (t > 0 && tid <= (int)mask) {
       before = look_back<8>(state + tid, RS_BINS, t, wait, [&](uint32_t tile) {
-        return (W)count_digit(io, (uint64_t)tile * RS_TILE, RS_TILE, shift, mask, (uint32_t)tid);
+        return (W)count_digit(io, tile, shift, mask, (uint32_t)tid);
       });
       st_relaxed(mine, P::PREFIX | (before + (W)cnt));
     }
@@ -1085,7 +1096,7 @@ int radix_passes(IO io, uint64_t n_host, const uint32_t* n_dev, int key_bits, co
   for (int p = 0; p < passes; ++p) {
     const int shift = p * dbits, nbits = std::min(dbits, key_bits - shift);
     const bool last = p + 1 == passes;
-    k_rs_pass<IO, W><<<grid, RS_THREADS, 0, st>>>(last ? io : io.plain(), n_host, n_dev, p, passes, shift, nbits, h,
+    k_rs_pass<IO, W><<<grid, RS_THREADS, 0, st>>>(last ? io : io.plain(), n_host, n_dev, p, shift, nbits, h,
                                                   state[p & 1], last ? nullptr : state[(p + 1) & 1],
                                                   last ? ranges : nullptr, num_ranges, base, sc.wait_cycles);
     swap(io);
@@ -1132,16 +1143,22 @@ int launch_radix_sort(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, ui
 int launch_radix_sort_pairs(uint2* p0, uint2* p1, uint64_t n_host, const uint32_t* n_dev, int key_bits,
                             const SortScratch& sc, int hdr, int* result_in_1, cudaStream_t st, uint2* ranges,
                             uint32_t num_ranges, bool zero_ranges, const unsigned long long* base, uint32_t* values) {
-  PairIO io{p0, p1, values};
-  auto swap = [](PairIO& x) {
-    PairIO y{x.out, const_cast<uint2*>(x.in), x.values};
-    x = y;
+  auto sort = [&](auto io) {
+    using IO = decltype(io);
+    auto swap = [](IO& x) {
+      IO y{x.out, const_cast<uint2*>(x.in), x.values};
+      x = y;
+    };
+    if (sc.wide)
+      return radix_passes<IO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges,
+                                                  num_ranges, base, zero_ranges);
+    return radix_passes<IO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges, num_ranges,
+                                      base, zero_ranges);
   };
-  if (sc.wide)
-    return radix_passes<PairIO, unsigned long long>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges,
-                                                    num_ranges, base, zero_ranges);
-  return radix_passes<PairIO, uint32_t>(io, n_host, n_dev, key_bits, sc, hdr, result_in_1, st, swap, ranges, num_ranges,
-                                        base, zero_ranges);
+  // Chunks where they can be met and gain; the kernels without them keep
+  // look-back's registers (65 against 63 us at 2.8 million).
+  if (key_bits > 8 && n_host >= RC_MIN) return sort(PairIO<true>{p0, p1, values});
+  return sort(PairIO<false>{p0, p1, values});
 }
 
 int launch_expand(const ExpandArgs& a, cudaStream_t st) {
