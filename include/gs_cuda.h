@@ -355,7 +355,10 @@ gs_status gs_raster_work(gs_rasterizer* r, uint64_t out[4], void* stream);
  * (32,0) selects the pixel-compacted kernels (one warp per tile spreading each
  * entry's box pixels over its lanes) for the colour-only persistent passes of
  * the training step; other passes fall back to (64,4) forward and (64,8)
- * backward. The backward with aux losses uses its own fixed shape.
+ * backward. The backward with aux losses uses its own fixed shape. Until
+ * shapes are tuned or set, the backward at tile 16 follows the launch's number
+ * of tiles: (64,1) below 4 per SM (below 6 in the persistent passes of the
+ * chosen form), (64,4) from 32 per SM on, (128,2) between.
  *
  * Autotuner (config-2 sweep of the batched form): at the handle's current
  * tile size, times the forward (projection + binning + raster) over every
@@ -378,11 +381,14 @@ gs_status gs_autotune_tiles(gs_rasterizer* r, const gs_camera* cams, uint32_t n_
                             void* stream, uint32_t out[5], float times_ms[6]);
 /* Applies launch shapes (the layout of gs_autotune's out, e.g. a stored
  * result) without timing. Each pair must be built for the handle's tile
- * size (table above), else GS_ERR_INVALID_ARG and nothing changes. Host-only. */
+ * size (table above), else GS_ERR_INVALID_ARG and nothing changes. The backward
+ * then keeps this shape whatever the number of tiles, also when it is the
+ * default's (128,2). Host-only. */
 gs_status gs_set_launch_shapes(gs_rasterizer* r, const uint32_t shapes[4]);
 /* Changes the tile edge (8, 16 or 32 pixels) of later forwards. Launch
  * shapes not built for the new size fall back to its first forward shape and
- * its default backward shape ((128,2) where built, else (64,4)). Tile rects,
+ * its default backward shape ((128,2) where built, else (64,4); at tile 16 by
+ * the number of tiles, as above). Tile rects,
  * entry lists, ranges and contributor indices of later forwards refer to the
  * new tiling (the oracle's rect arithmetic takes the tile size as a
  * parameter). GS_ERR_INVALID_ARG for other sizes, or for a tile other than

@@ -367,14 +367,23 @@ void default_bwd_shape(gs_rasterizer* r) {
 
 // The backward's shape for a launch over `tiles` tiles. While neither
 // gs_set_launch_shapes nor the autotuner chose one, tiles of 16 pixels take 8
-// warps each when there are few (the longest tile decides: 758 tiles 1504 ->
-// 1387 us a step, 800 tiles 539 -> 507) and 2 warps of 4 pixels a thread when
-// there are many (throughput decides: 5700 tiles 1509 -> 1395, 8160 tiles
-// 5139 -> 4865).
-RasterShape bwd_shape(const gs_rasterizer* r, int tiles) {
+// warps each when there are few (the longest tile decides) and 2 warps of 4
+// pixels a thread when there are many (throughput decides). Kernel time of
+// (64, 1) against (128, 2), on scenes of 16 and 100 thousand surfels spread
+// evenly and 40 and 200 thousand in clusters (whose longest tiles are far longer
+// than the mean): up to 3.2 tiles an SM 3 % slower to 25 % faster in every form.
+// One launch a tile: 4.0 an SM 216 and 224, 294 and 369, 376 and 365, 863 and 885
+// us for the four; 6.1 an SM 210 and 244, 281 and 431, 355 and 383, 663 and 835.
+// Persistent, heaviest tile first: 5.1 an SM 188 and 155, 216 and 252, 314 and
+// 262, 537 and 460; 7.8 an SM 201 and 292 (100 thousand), 425 and 477 (200).
+// (64, 4) against (128, 2), 100 and 200 thousand surfels, persistent and not: 24
+// an SM 290 and 259, 445 and 473, 497 and 493, 832 and 938; 31.5 an SM 428 and
+// 358, 621 and 558, 654 and 515, 1021 and 942; 55 an SM 474 and 382, 665 and 595,
+// 840 and 644, 1258 and 1095.
+RasterShape bwd_shape(const gs_rasterizer* r, int tiles, bool persistent) {
   RasterShape s{r->bwd_batch, r->bwd_ppt};
   if (r->bwd_auto && r->tile == 16) {
-    if (tiles < 8 * r->num_sms) s = {64, 1};
+    if (tiles < (persistent ? 6 : 4) * r->num_sms) s = {64, 1};
     else if (tiles >= 32 * r->num_sms) s = {64, 4};
   }
   return s;
@@ -561,7 +570,7 @@ gs_status run_backward_raster(gs_rasterizer* r, const ViewInfo* vdev, uint32_t n
     ra.mask = r->mask;
     ra.mask_off = r->mask_off;
   }
-  const RasterShape sh = bwd_shape(r, tiles);
+  const RasterShape sh = bwd_shape(r, tiles, persistent);
   int grid = tiles;
   if (persistent) {
     TRY_CUDA(r, cudaMemsetAsync(r->words + 3, 0, sizeof(uint32_t), st));

@@ -1,7 +1,7 @@
-"""The backward raster's shape as the number of tiles chooses it (below 8 and
-from 32 tiles per SM on, and between) against a fixed shape: the same
-gradients up to the order of float sums (bound: f32 tolerance of a step,
-2e-4 in the 2-norm)."""
+"""The backward raster's shape as the number of tiles chooses it (below 4, or 6
+in the persistent form, and from 32 tiles per SM on, and between) against a
+fixed shape: the same gradients up to the order of float sums (bound: f32
+tolerance of a step, 2e-4 in the 2-norm)."""
 import numpy as np
 import pytest
 
@@ -13,10 +13,12 @@ pytestmark = pytest.mark.gpu
 WIDTHS = {"grad_pos": 4, "grad_scales": 2, "grad_quat": 4, "grad_opacity": 1, "grad_sh": 48}
 
 
-@pytest.mark.parametrize("W,H", [(64, 48), (16 * 37, 16 * 31), (16 * 37, 16 * 32), (16 * 37, 16 * 33), (1184, 16 * 63),
-                                 (1184, 16 * 64), (1183, 1039)])
+@pytest.mark.parametrize("W,H", [(64, 48), (16 * 37, 16 * 15), (16 * 37, 16 * 16), (16 * 37, 16 * 17),
+                                 (16 * 37, 16 * 23), (16 * 37, 16 * 24), (16 * 37, 16 * 31), (16 * 37, 16 * 32),
+                                 (16 * 37, 16 * 33), (1184, 16 * 63), (1184, 16 * 64), (1183, 1039)])
 @pytest.mark.parametrize("deterministic", [False, True])
-def test_chosen_by_tiles_equals_fixed(W, H, deterministic):
+@pytest.mark.parametrize("persistent", [False, True])
+def test_chosen_by_tiles_equals_fixed(W, H, deterministic, persistent):
     scene, cam = make_scene(404, 2000, 1, 128)
     cam.focal *= W / cam.width
     cam.width, cam.height = W, H
@@ -25,7 +27,8 @@ def test_chosen_by_tiles_equals_fixed(W, H, deterministic):
     w[:, 3] = 0
     got = []
     for fixed in (False, True):
-        r = Rasterizer(scene.n, W, H, 4096 * scene.n, color_only=True, deterministic=deterministic)
+        r = Rasterizer(scene.n, W, H, 4096 * scene.n, color_only=True, deterministic=deterministic,
+                       persistent=persistent)
         if fixed:
             r.set_launch_shapes(128, 1, 128, 2)
         r.upload_scene(scene_input(scene))
