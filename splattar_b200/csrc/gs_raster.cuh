@@ -421,9 +421,6 @@ __device__ __forceinline__ void cut_tile_end(const RasterArgs& a, int tile, uint
 // CTAs (72 registers) and 3.32 → 4.21 ms earlier between 72 registers and
 // the compiler's 99. With the per-entry hit forms the walk needs fewer live
 // values; before them 64 registers ran slower than 72.
-#ifndef GS_FWD_UNROLL
-#define GS_FWD_UNROLL 2
-#endif
 #ifndef GS_FWD_2WARP_CTAS
 #define GS_FWD_2WARP_CTAS 16
 #endif
@@ -444,7 +441,9 @@ __global__ void __launch_bounds__(TS * TS / PPT, ((TS * TS / PPT) == 64 && COLOR
   constexpr bool GM = COLOR && !MASK && TS == 16;
   constexpr int GPL = PPT >= 8 ? 2 : 1;              // row groups per lane
   constexpr int GW = (BATCH + 31) / 32;              // 32-entry words per batch
-  constexpr int FWD_U = PPT == 1 && !MASK ? GS_FWD_UNROLL : 1;  // entries evaluated side by side
+  // Entries evaluated side by side: two at one pixel per thread, whose walk is
+  // one serial chain; more pixels per thread are independent work already.
+  constexpr int FWD_U = PPT == 1 && !MASK ? 2 : 1;
   __shared__ float4 s_r0[BATCH], s_r1[BATCH], s_r2[BATCH], s_r3[BATCH];
   __shared__ uint2 s_msk[BATCH];  // box_masks of the staged entry
   __shared__ float4 s_r4[COLOR ? 1 : BATCH];
@@ -577,170 +576,171 @@ __global__ void __launch_bounds__(TS * TS / PPT, ((TS * TS / PPT) == 64 && COLOR
         uint32_t sel = __ballot_sync(FULL, (lm.x & lrows) != 0u && (lm.y & lcols) != 0u);
         const bool walked = sel != 0u;
         if constexpr (FWD_U > 1) {
-        while (sel) {
-          // FWD_U entries' hits are evaluated side by side, then composited in
-          // list order: a pixel's chain of one entry after another is then T
-          // alone instead of the whole hit test.
-          int ks[FWD_U];
-          bool on[FWD_U];
-          uint32_t fm = RAYBIT | FARBIT;
-          float4 e3[FWD_U];
-          float al[FWD_U], ht[FWD_U];
-          uint2 mk[FWD_U];
-#pragma unroll
-          for (int u = 0; u < FWD_U; ++u) {
-            on[u] = sel != 0u;
-            ks[u] = on[u] ? wd + __ffs(sel) - 1 : ks[0];
-            sel &= sel - 1u;
-            mk[u] = s_msk[ks[u]];
-            fm &= mk[u].y;
-          }
-          auto hits = [&](auto ray_tag) {
-            constexpr int FAST = decltype(ray_tag)::value;
+          while (sel) {
+            // FWD_U entries' hits are evaluated side by side, then composited in
+            // list order: a pixel's chain of one entry after another is then T
+            // alone instead of the whole hit test.
+            int ks[FWD_U];
+            bool on[FWD_U];
+            uint32_t fm = RAYBIT | FARBIT;
+            float4 e3[FWD_U];
+            float al[FWD_U], ht[FWD_U];
+            uint2 mk[FWD_U];
 #pragma unroll
             for (int u = 0; u < FWD_U; ++u) {
-              const int k = ks[u];
-              const float4 r0 = s_r0[k], r1 = s_r1[k], r2 = s_r2[k];
-              e3[u] = s_r3[k];
-              const ColPart cp = col_part(r0, r1, r2, g.sx, g.kx);
-              const Hit h = eval_hit<FAST>(cp, r0, r1, r2, COLOR ? 0.f : s_r4[COLOR ? 0 : k].w, g.sy[0], g.ky[0]);
-              const float alpha =
-                  FAST ? __fmul_rn(e3[u].w, h.ghat) : fminf(__fmul_rn(e3[u].w, h.ghat), ALPHA_CLAMP);
-              const bool take = on[u] && ((mk[u].y >> L::col(tid)) & 1u) && ((mk[u].x >> L::row(tid)) & 1u) &&
-                                !(alpha < ALPHA_SKIP);
-              al[u] = take ? alpha : 0.f;
-              ht[u] = h.t;
+              on[u] = sel != 0u;
+              ks[u] = on[u] ? wd + __ffs(sel) - 1 : ks[0];
+              sel &= sel - 1u;
+              mk[u] = s_msk[ks[u]];
+              fm &= mk[u].y;
             }
-          };
-          if (fm & FARBIT) hits(std::integral_constant<int, HIT_RAY_FAR>{});
-          else if (fm & RAYBIT) hits(std::integral_constant<int, HIT_RAY_OK>{});
-          else hits(std::integral_constant<int, HIT_FULL>{});
+            auto hits = [&](auto ray_tag) {
+              constexpr int FAST = decltype(ray_tag)::value;
 #pragma unroll
-          for (int u = 0; u < FWD_U; ++u) {
-            if (al[u] > 0.f && !dm) {
-              const float w = T[0] * al[u];
-              cr[0] += e3[u].x * w; cg[0] += e3[u].y * w; cb[0] += e3[u].z * w;
-              aa[0] += w;
-              if (!COLOR) {
-                const float4 r4 = s_r4[COLOR ? 0 : ks[u]];
-                ad[0] += ht[u] * w;
-                nx[0] += r4.x * w; ny[0] += r4.y * w; nz[0] += r4.z * w;
+              for (int u = 0; u < FWD_U; ++u) {
+                const int k = ks[u];
+                const float4 r0 = s_r0[k], r1 = s_r1[k], r2 = s_r2[k];
+                e3[u] = s_r3[k];
+                const ColPart cp = col_part(r0, r1, r2, g.sx, g.kx);
+                const Hit h = eval_hit<FAST>(cp, r0, r1, r2, COLOR ? 0.f : s_r4[COLOR ? 0 : k].w, g.sy[0], g.ky[0]);
+                const float alpha =
+                    FAST ? __fmul_rn(e3[u].w, h.ghat) : fminf(__fmul_rn(e3[u].w, h.ghat), ALPHA_CLAMP);
+                const bool take = on[u] && ((mk[u].y >> L::col(tid)) & 1u) && ((mk[u].x >> L::row(tid)) & 1u) &&
+                                  !(alpha < ALPHA_SKIP);
+                al[u] = take ? alpha : 0.f;
+                ht[u] = h.t;
               }
-              T[0] = __fmul_rn(T[0], 1.0f - al[u]);
-              nc[0] = base - range.x + (uint32_t)s_j[ks[u]] + 1u;
-              if (GM) gcur[0] |= 1u << (ks[u] & 31);
-              if (T[0] < T_TERMINATE) dm = 1u;
-            }
-          }
-          if (__all_sync(FULL, dm != 0u)) break;
-        }
-        tdone = dm == PMASK;
-        }
-        while (sel && FWD_U == 1) {
-          const int k = wd + __ffs(sel) - 1;
-          sel &= sel - 1u;
-          const uint32_t kbit = 1u << (k & 31);
-          const uint2 mk = s_msk[k];
-          // need: bit p when pixel p is live and inside the entry's α-box
-          const uint32_t need = ((mk.y >> L::col(tid)) & 1u) ? (mk.x >> L::row(tid)) & ~dm & PMASK : 0u;
-          if (need) {
-            const float4 r0 = s_r0[k], r1 = s_r1[k], r2 = s_r2[k];
-            const float4 r3 = s_r3[k];
-            const float4 r4 = COLOR ? make_float4(0.f, 0.f, 0.f, 0.f) : s_r4[k];
-            const uint32_t idx1 = base - range.x + (uint32_t)s_j[k] + 1u;
-            const ColPart cp = col_part(r0, r1, r2, g.sx, g.kx);
-            constexpr int PS = PPT >= 2 ? 2 : 1;  // pixels per hit evaluation
-            // the pixel walk, with or without the per-pixel ray test
-            auto walk = [&](auto ray_tag) {
-            constexpr int FAST = decltype(ray_tag)::value;
-#pragma unroll
-            for (int pp = 0; pp < PPT; pp += PS) {
-            bool need_q[PS];
-            Hit hh[PS];
-#pragma unroll
-            for (int q = 0; q < PS; ++q) need_q[q] = (need >> (pp + q)) & 1u;
-            if constexpr (PS == 2) {
-              if (!((need >> pp) & 3u)) continue;
-              eval_hit2<FAST>(cp, r0, r1, r2, r4.w, make_float2(g.sy[pp], g.sy[pp + 1]),
-                                make_float2(g.ky[pp], g.ky[pp + 1]), hh[0], hh[PS - 1]);
-            } else {
-              if (!need_q[0]) continue;
-              hh[0] = eval_hit<FAST>(cp, r0, r1, r2, r4.w, g.sy[pp], g.ky[pp]);
-            }
-            if constexpr (PS == 2 && COLOR && !MASK && PPT <= 4) {  // (8 pixels per thread would spill)
-              // Both pixels of the pair composited at once in packed FP32: a
-              // pixel that does not take the entry gets α = 0, so its weight is
-              // 0 and its T is multiplied by 1 (both exact); each component
-              // rounds as the scalar code below would.
-              // (fast form: opacity < ALPHA_CLAMP and ĝ ≤ 1, so the clamp never acts)
-              const float a0 = FAST ? __fmul_rn(r3.w, hh[0].ghat) : fminf(__fmul_rn(r3.w, hh[0].ghat), ALPHA_CLAMP);
-              const float a1 = FAST ? __fmul_rn(r3.w, hh[PS - 1].ghat)
-                                    : fminf(__fmul_rn(r3.w, hh[PS - 1].ghat), ALPHA_CLAMP);
-              const bool c0 = need_q[0] && !(a0 < ALPHA_SKIP), c1 = need_q[PS - 1] && !(a1 < ALPHA_SKIP);
-              if (c0 || c1) {
-                const float2 al = make_float2(c0 ? a0 : 0.f, c1 ? a1 : 0.f);
-                const float2 Tp = make_float2(T[pp], T[pp + 1]);
-                const float2 w = __fmul2_rn(Tp, al);
-                float2 vr = __ffma2_rn(make_float2(r3.x, r3.x), w, make_float2(cr[pp], cr[pp + 1]));
-                float2 vg = __ffma2_rn(make_float2(r3.y, r3.y), w, make_float2(cg[pp], cg[pp + 1]));
-                float2 vb = __ffma2_rn(make_float2(r3.z, r3.z), w, make_float2(cb[pp], cb[pp + 1]));
-                float2 va = __fadd2_rn(make_float2(aa[pp], aa[pp + 1]), w);
-                const float2 Tn = __fmul2_rn(Tp, __fadd2_rn(make_float2(1.0f, 1.0f), make_float2(-al.x, -al.y)));
-                cr[pp] = vr.x; cr[pp + 1] = vr.y; cg[pp] = vg.x; cg[pp + 1] = vg.y;
-                cb[pp] = vb.x; cb[pp + 1] = vb.y; aa[pp] = va.x; aa[pp + 1] = va.y;
-                T[pp] = Tn.x; T[pp + 1] = Tn.y;
-                // both pixels of a pair lie in one 4-row group (a thread's first row is even)
-                if (GM) gcur[(((L::row(tid) & 3) + pp) >> 2) & (GPL - 1)] |= kbit;
-                if (c0) {
-                  nc[pp] = idx1;
-                  if (Tn.x < T_TERMINATE) dm |= 1u << pp;
-                }
-                if (c1) {
-                  nc[pp + 1] = idx1;
-                  if (Tn.y < T_TERMINATE) dm |= 2u << pp;
-                }
-              }
-              continue;
-            }
-#pragma unroll
-            for (int q = 0; q < PS; ++q) {
-              const int p = pp + q;
-              if (!need_q[q]) continue;
-              const Hit& h = hh[q];
-              const float alpha = FAST ? __fmul_rn(r3.w, h.ghat) : fminf(__fmul_rn(r3.w, h.ghat), ALPHA_CLAMP);
-              if (alpha < ALPHA_SKIP) continue;
-              const float w = T[p] * alpha;
-              cr[p] += r3.x * w; cg[p] += r3.y * w; cb[p] += r3.z * w;
-              aa[p] += w;
-              if (!COLOR) {
-                ad[p] += h.t * w;
-                nx[p] += r4.x * w; ny[p] += r4.y * w; nz[p] += r4.z * w;
-              }
-              T[p] = __fmul_rn(T[p], 1.0f - alpha);
-              nc[p] = idx1;
-              if (GM) gcur[(((L::row(tid) & 3) + p) >> 2) & (GPL - 1)] |= kbit;
-              if (masks) {
-                const uint32_t cidx = idx1 - 1u;
-                const int w = (int)(cidx >> 5);
-                if (w != mi[p]) {  // close the current word, zero the words skipped
-                  uint32_t* m = a.mask + mbase + mpix + p * TS;
-                  m[(size_t)mi[p] * TP] = mw[p];
-                  for (int z = mi[p] + 1; z < w; ++z) m[(size_t)z * TP] = 0u;
-                  mi[p] = w;
-                  mw[p] = 0u;
-                }
-                mw[p] |= 1u << (cidx & 31u);
-              }
-              if (T[p] < T_TERMINATE) dm |= 1u << p;
-            }
-            }
             };
-            if (RAYFLAG && (mk.y & FARBIT)) walk(std::integral_constant<int, HIT_RAY_FAR>{});
-            else if (RAYFLAG && (mk.y & RAYBIT)) walk(std::integral_constant<int, HIT_RAY_OK>{});
-            else walk(std::integral_constant<int, HIT_FULL>{});
-            tdone = dm == PMASK;
+            if (fm & FARBIT) hits(std::integral_constant<int, HIT_RAY_FAR>{});
+            else if (fm & RAYBIT) hits(std::integral_constant<int, HIT_RAY_OK>{});
+            else hits(std::integral_constant<int, HIT_FULL>{});
+#pragma unroll
+            for (int u = 0; u < FWD_U; ++u) {
+              if (al[u] > 0.f && !dm) {
+                const float w = T[0] * al[u];
+                cr[0] += e3[u].x * w; cg[0] += e3[u].y * w; cb[0] += e3[u].z * w;
+                aa[0] += w;
+                if (!COLOR) {
+                  const float4 r4 = s_r4[COLOR ? 0 : ks[u]];
+                  ad[0] += ht[u] * w;
+                  nx[0] += r4.x * w; ny[0] += r4.y * w; nz[0] += r4.z * w;
+                }
+                T[0] = __fmul_rn(T[0], 1.0f - al[u]);
+                nc[0] = base - range.x + (uint32_t)s_j[ks[u]] + 1u;
+                if (GM) gcur[0] |= 1u << (ks[u] & 31);
+                if (T[0] < T_TERMINATE) dm = 1u;
+              }
+            }
+            if (__all_sync(FULL, dm != 0u)) break;
           }
-          if (__all_sync(FULL, tdone)) break;
+          tdone = dm == PMASK;
+        } else {
+          while (sel) {
+            const int k = wd + __ffs(sel) - 1;
+            sel &= sel - 1u;
+            const uint32_t kbit = 1u << (k & 31);
+            const uint2 mk = s_msk[k];
+            // need: bit p when pixel p is live and inside the entry's α-box
+            const uint32_t need = ((mk.y >> L::col(tid)) & 1u) ? (mk.x >> L::row(tid)) & ~dm & PMASK : 0u;
+            if (need) {
+              const float4 r0 = s_r0[k], r1 = s_r1[k], r2 = s_r2[k];
+              const float4 r3 = s_r3[k];
+              const float4 r4 = COLOR ? make_float4(0.f, 0.f, 0.f, 0.f) : s_r4[k];
+              const uint32_t idx1 = base - range.x + (uint32_t)s_j[k] + 1u;
+              const ColPart cp = col_part(r0, r1, r2, g.sx, g.kx);
+              constexpr int PS = PPT >= 2 ? 2 : 1;  // pixels per hit evaluation
+              // the pixel walk, with or without the per-pixel ray test
+              auto walk = [&](auto ray_tag) {
+              constexpr int FAST = decltype(ray_tag)::value;
+#pragma unroll
+              for (int pp = 0; pp < PPT; pp += PS) {
+              bool need_q[PS];
+              Hit hh[PS];
+#pragma unroll
+              for (int q = 0; q < PS; ++q) need_q[q] = (need >> (pp + q)) & 1u;
+              if constexpr (PS == 2) {
+                if (!((need >> pp) & 3u)) continue;
+                eval_hit2<FAST>(cp, r0, r1, r2, r4.w, make_float2(g.sy[pp], g.sy[pp + 1]),
+                                  make_float2(g.ky[pp], g.ky[pp + 1]), hh[0], hh[PS - 1]);
+              } else {
+                if (!need_q[0]) continue;
+                hh[0] = eval_hit<FAST>(cp, r0, r1, r2, r4.w, g.sy[pp], g.ky[pp]);
+              }
+              if constexpr (PS == 2 && COLOR && !MASK && PPT <= 4) {  // (8 pixels per thread would spill)
+                // Both pixels of the pair composited at once in packed FP32: a
+                // pixel that does not take the entry gets α = 0, so its weight is
+                // 0 and its T is multiplied by 1 (both exact); each component
+                // rounds as the scalar code below would.
+                // (fast form: opacity < ALPHA_CLAMP and ĝ ≤ 1, so the clamp never acts)
+                const float a0 = FAST ? __fmul_rn(r3.w, hh[0].ghat) : fminf(__fmul_rn(r3.w, hh[0].ghat), ALPHA_CLAMP);
+                const float a1 = FAST ? __fmul_rn(r3.w, hh[PS - 1].ghat)
+                                      : fminf(__fmul_rn(r3.w, hh[PS - 1].ghat), ALPHA_CLAMP);
+                const bool c0 = need_q[0] && !(a0 < ALPHA_SKIP), c1 = need_q[PS - 1] && !(a1 < ALPHA_SKIP);
+                if (c0 || c1) {
+                  const float2 al = make_float2(c0 ? a0 : 0.f, c1 ? a1 : 0.f);
+                  const float2 Tp = make_float2(T[pp], T[pp + 1]);
+                  const float2 w = __fmul2_rn(Tp, al);
+                  float2 vr = __ffma2_rn(make_float2(r3.x, r3.x), w, make_float2(cr[pp], cr[pp + 1]));
+                  float2 vg = __ffma2_rn(make_float2(r3.y, r3.y), w, make_float2(cg[pp], cg[pp + 1]));
+                  float2 vb = __ffma2_rn(make_float2(r3.z, r3.z), w, make_float2(cb[pp], cb[pp + 1]));
+                  float2 va = __fadd2_rn(make_float2(aa[pp], aa[pp + 1]), w);
+                  const float2 Tn = __fmul2_rn(Tp, __fadd2_rn(make_float2(1.0f, 1.0f), make_float2(-al.x, -al.y)));
+                  cr[pp] = vr.x; cr[pp + 1] = vr.y; cg[pp] = vg.x; cg[pp + 1] = vg.y;
+                  cb[pp] = vb.x; cb[pp + 1] = vb.y; aa[pp] = va.x; aa[pp + 1] = va.y;
+                  T[pp] = Tn.x; T[pp + 1] = Tn.y;
+                  // both pixels of a pair lie in one 4-row group (a thread's first row is even)
+                  if (GM) gcur[(((L::row(tid) & 3) + pp) >> 2) & (GPL - 1)] |= kbit;
+                  if (c0) {
+                    nc[pp] = idx1;
+                    if (Tn.x < T_TERMINATE) dm |= 1u << pp;
+                  }
+                  if (c1) {
+                    nc[pp + 1] = idx1;
+                    if (Tn.y < T_TERMINATE) dm |= 2u << pp;
+                  }
+                }
+                continue;
+              }
+#pragma unroll
+              for (int q = 0; q < PS; ++q) {
+                const int p = pp + q;
+                if (!need_q[q]) continue;
+                const Hit& h = hh[q];
+                const float alpha = FAST ? __fmul_rn(r3.w, h.ghat) : fminf(__fmul_rn(r3.w, h.ghat), ALPHA_CLAMP);
+                if (alpha < ALPHA_SKIP) continue;
+                const float w = T[p] * alpha;
+                cr[p] += r3.x * w; cg[p] += r3.y * w; cb[p] += r3.z * w;
+                aa[p] += w;
+                if (!COLOR) {
+                  ad[p] += h.t * w;
+                  nx[p] += r4.x * w; ny[p] += r4.y * w; nz[p] += r4.z * w;
+                }
+                T[p] = __fmul_rn(T[p], 1.0f - alpha);
+                nc[p] = idx1;
+                if (GM) gcur[(((L::row(tid) & 3) + p) >> 2) & (GPL - 1)] |= kbit;
+                if (masks) {
+                  const uint32_t cidx = idx1 - 1u;
+                  const int w = (int)(cidx >> 5);
+                  if (w != mi[p]) {  // close the current word, zero the words skipped
+                    uint32_t* m = a.mask + mbase + mpix + p * TS;
+                    m[(size_t)mi[p] * TP] = mw[p];
+                    for (int z = mi[p] + 1; z < w; ++z) m[(size_t)z * TP] = 0u;
+                    mi[p] = w;
+                    mw[p] = 0u;
+                  }
+                  mw[p] |= 1u << (cidx & 31u);
+                }
+                if (T[p] < T_TERMINATE) dm |= 1u << p;
+              }
+              }
+              };
+              if (RAYFLAG && (mk.y & FARBIT)) walk(std::integral_constant<int, HIT_RAY_FAR>{});
+              else if (RAYFLAG && (mk.y & RAYBIT)) walk(std::integral_constant<int, HIT_RAY_OK>{});
+              else walk(std::integral_constant<int, HIT_FULL>{});
+              tdone = dm == PMASK;
+            }
+            if (__all_sync(FULL, tdone)) break;
+          }
         }
         if (GM && gm_on && walked) flush_row_groups<PPT, GPL, GM ? GW : 1>(gcur, s_gw, g0, wd >> 5);
       }
