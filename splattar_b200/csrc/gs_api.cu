@@ -207,7 +207,6 @@ struct gs_rasterizer {
 struct gs_binner {
   uint32_t max_items = 0, num_tiles = 0;
   uint64_t max_entries = 0;
-  uint4* rects_tmp = nullptr;  // unused: rects come from the caller
   uint32_t* counts = nullptr;  // the allocation of this and the next five members
   uint32_t* sorted_counts = nullptr;  // counts in depth order
   uint32_t* ref_offsets = nullptr;
@@ -220,8 +219,6 @@ struct gs_binner {
   uint2* ranges = nullptr;
   unsigned long long* total = nullptr;
   uint32_t* words = nullptr;
-  int ent_in1 = 0;
-  void* scan_scratch = nullptr;
   void* sort_scratch = nullptr;
   SortScratch sort{};  // layout of sort_scratch
 };
@@ -2060,7 +2057,7 @@ extern "C" gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, ui
     const gs_status s = pool_alloc(&scan, scan_scratch_bytes(), st);
     if (s) return s;
   }
-  int e = launch_scan(in, nullptr, out, n, nullptr, total_dev, nullptr, scan, st);
+  int e = launch_scan(in, out, n, nullptr, total_dev, scan, st);
   if (!captured) cudaFreeAsync(scan, st);
   if (e) return fail(nullptr, GS_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
   return GS_OK;

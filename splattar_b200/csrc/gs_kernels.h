@@ -178,15 +178,14 @@ int launch_raster_bwd(const RasterArgs& a, int tile, int prec, bool aux, int ppt
                       bool persistent, int grid, cudaStream_t st);
 
 // ---- sort / scan / binning (gs_sort.cu) ----
-// Exclusive scan of n u32 values read as in[perm ? perm[i] : i] (n from
-// n_dev when non-null, else n_host) in three launches that wait for nothing
-// and need scan_scratch_bytes() of scratch whatever n is: the public scan,
-// densify, MCMC and the stored-state masks. Writes out[i], and the total to
-// total_u32 (saturated) / total_u64 when non-null.
+// Exclusive scan of n u32 values (n from n_dev when non-null, else n_host) in
+// three launches that wait for nothing and need scan_scratch_bytes() of
+// scratch whatever n is: the public scan, densify, MCMC and the stored-state
+// masks. Writes out[i], and the total to total_u32 (saturated) when non-null.
 constexpr int SCAN_GRID = 512;  // blocks of the chunked scan
 size_t scan_scratch_bytes();
-int launch_scan(const uint32_t* in, const uint32_t* perm, uint32_t* out, uint64_t n_host, const uint32_t* n_dev,
-                uint32_t* total_u32, unsigned long long* total_u64, void* scratch, cudaStream_t st);
+int launch_scan(const uint32_t* in, uint32_t* out, uint64_t n_host, const uint32_t* n_dev, uint32_t* total_u32,
+                void* scratch, cudaStream_t st);
 
 constexpr int RS_TILE = 4096;   // elements per tile of a sort pass
 constexpr int RS_SMALL = 8192;  // up to this many elements one block sorts in shared memory

@@ -342,7 +342,7 @@ int launch_mcmc_relocate(McmcArgs& a, int prec, void* scan_scratch, const SortSc
   const int g = grid_n(a.n);
   cudaMemsetAsync(a.counters, 0, sizeof(uint32_t) * 8, st);
   k_mcmc_flags<<<g, 256, 0, st>>>(a);
-  int e = launch_scan(a.dead, nullptr, a.dead_rank, a.n, nullptr, a.counters + 0, nullptr, scan_scratch, st);
+  int e = launch_scan(a.dead, a.dead_rank, a.n, nullptr, a.counters + 0, scan_scratch, st);
   if (e) return e;
   auto* bsum = reinterpret_cast<unsigned long long*>(scan_scratch);
   k_scan64_reduce<<<SCAN_GRID, 256, 0, st>>>(a.weight, a.n, bsum);
@@ -358,15 +358,14 @@ int launch_mcmc_relocate(McmcArgs& a, int prec, void* scan_scratch, const SortSc
     if (e) return e;
     a.sorted_size_key = in1 ? a.key2 : a.size_key;
     k_mcmc_over_flags<<<g, 256, 0, st>>>(a);
-    e = launch_scan(a.over_flag, nullptr, a.over_rank, a.n, nullptr, a.counters + 5, nullptr, scan_scratch, st);
+    e = launch_scan(a.over_flag, a.over_rank, a.n, nullptr, a.counters + 5, scan_scratch, st);
     if (e) return e;
     k_mcmc_over_list<<<g, 256, 0, st>>>(a);
     // The size keys are consumed; their buffers take the second sort.
     e = launch_radix_sort(a.over_key, a.over_val, a.key2, a.val2, a.n, a.counters + 5, 32, sc, 1, &in1, st);
     if (e) return e;
     a.over_sorted_val = in1 ? a.val2 : a.over_val;
-    e = launch_scan(a.leftover_flag, nullptr, a.left_rank, a.n, a.counters + 0, a.counters + 6, nullptr, scan_scratch,
-                    st);
+    e = launch_scan(a.leftover_flag, a.left_rank, a.n, a.counters + 0, a.counters + 6, scan_scratch, st);
     if (e) return e;
     k_mcmc_left_list<<<g, 256, 0, st>>>(a);
     k_mcmc_split_count<<<1, 1, 0, st>>>(a);

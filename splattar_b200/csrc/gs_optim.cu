@@ -170,9 +170,9 @@ int launch_densify(DensifyArgs& a, void* scan_scratch, cudaStream_t st) {
   uint32_t* n_keep = a.n_out_dev + 1;
   uint32_t* n_clone = a.n_out_dev + 2;
   k_densify_flags<<<grid_of(a.n), 256, 0, st>>>(a, keep, clone);
-  int e = launch_scan(keep, nullptr, keep_off, a.n, nullptr, n_keep, nullptr, scan_scratch, st);
+  int e = launch_scan(keep, keep_off, a.n, nullptr, n_keep, scan_scratch, st);
   if (e) return e;
-  e = launch_scan(clone, nullptr, clone_off, a.n, nullptr, n_clone, nullptr, scan_scratch, st);
+  e = launch_scan(clone, clone_off, a.n, nullptr, n_clone, scan_scratch, st);
   if (e) return e;
   k_densify_count<<<1, 1, 0, st>>>(n_keep, n_clone, a.capacity, a.n_out_dev);
   for (int k = 0; k < a.n_arrays; ++k) {

@@ -47,39 +47,30 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-__device__ __forceinline__ uint32_t scan_in(const uint32_t* in, const uint32_t* perm, uint64_t i) {
-  return perm ? in[perm[i]] : in[i];
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* in, const uint32_t* perm, uint64_t n_host,
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* in, uint64_t n_host,
                                                               const uint32_t* n_dev, unsigned long long* bsum) {
   const uint64_t n = read_n(n_host, n_dev);
   const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const uint64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   unsigned long long s = 0;
-  for (uint64_t i = beg + threadIdx.x; i < end; i += SCAN_THREADS) s += scan_in(in, perm, i);
+  for (uint64_t i = beg + threadIdx.x; i < end; i += SCAN_THREADS) s += in[i];
   using BR = cub::BlockReduce<unsigned long long, SCAN_THREADS>;
   __shared__ typename BR::TempStorage tmp;
   s = BR(tmp).Sum(s);
   if (threadIdx.x == 0) bsum[blockIdx.x] = s;
 }
 
-__global__ void __launch_bounds__(SCAN_GRID) k_scan_blocks(unsigned long long* bsum, uint32_t* total_u32,
-                                                           unsigned long long* total_u64) {
+__global__ void __launch_bounds__(SCAN_GRID) k_scan_blocks(unsigned long long* bsum, uint32_t* total_u32) {
   using BS = cub::BlockScan<unsigned long long, SCAN_GRID>;
   __shared__ typename BS::TempStorage tmp;
   unsigned long long v = bsum[threadIdx.x], excl, agg;
   BS(tmp).ExclusiveSum(v, excl, agg);
   bsum[threadIdx.x] = excl;
-  if (threadIdx.x == 0) {
-    if (total_u32) *total_u32 = agg > 0xffffffffull ? 0xffffffffu : (uint32_t)agg;
-    if (total_u64) *total_u64 = agg;
-  }
+  if (threadIdx.x == 0 && total_u32) *total_u32 = agg > 0xffffffffull ? 0xffffffffu : (uint32_t)agg;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, const uint32_t* perm, uint32_t* out,
-                                                            uint64_t n_host, const uint32_t* n_dev,
-                                                            const unsigned long long* boff) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, uint32_t* out, uint64_t n_host,
+                                                            const uint32_t* n_dev, const unsigned long long* boff) {
   const uint64_t n = read_n(n_host, n_dev);
   const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const uint64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
@@ -92,7 +83,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* in, 
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
       const uint64_t i = t0 + (uint64_t)threadIdx.x * SCAN_ITEMS + k;
-      v[k] = i < end ? scan_in(in, perm, i) : 0u;
+      v[k] = i < end ? in[i] : 0u;
       loc += v[k];
     }
     uint32_t excl, agg;
@@ -713,6 +704,10 @@ __global__ void __launch_bounds__(NT) k_rs_small(SplitIO io, int n, int passes, 
 }
 
 // -------------------------------------------------------------- entry scan
+__device__ __forceinline__ uint32_t scan_in(const uint32_t* in, const uint32_t* perm, uint64_t i) {
+  return perm ? in[perm[i]] : in[i];
+}
+
 // Exclusive scan of the items' tile counts in one pass over tiles of
 // ES_TILE, and the entry-capacity guard: when the scene needs more entries
 // than were allocated (base + total > capacity), the totals are set to zero
@@ -1062,12 +1057,12 @@ int grid_for(uint64_t n_max, int per_block, int cap_blocks) {
 
 size_t scan_scratch_bytes() { return sizeof(unsigned long long) * SCAN_GRID; }
 
-int launch_scan(const uint32_t* in, const uint32_t* perm, uint32_t* out, uint64_t n_host, const uint32_t* n_dev,
-                uint32_t* total_u32, unsigned long long* total_u64, void* scratch, cudaStream_t st) {
+int launch_scan(const uint32_t* in, uint32_t* out, uint64_t n_host, const uint32_t* n_dev, uint32_t* total_u32,
+                void* scratch, cudaStream_t st) {
   auto* bsum = reinterpret_cast<unsigned long long*>(scratch);
-  k_scan_reduce<<<SCAN_GRID, SCAN_THREADS, 0, st>>>(in, perm, n_host, n_dev, bsum);
-  k_scan_blocks<<<1, SCAN_GRID, 0, st>>>(bsum, total_u32, total_u64);
-  k_scan_down<<<SCAN_GRID, SCAN_THREADS, 0, st>>>(in, perm, out, n_host, n_dev, bsum);
+  k_scan_reduce<<<SCAN_GRID, SCAN_THREADS, 0, st>>>(in, n_host, n_dev, bsum);
+  k_scan_blocks<<<1, SCAN_GRID, 0, st>>>(bsum, total_u32);
+  k_scan_down<<<SCAN_GRID, SCAN_THREADS, 0, st>>>(in, out, n_host, n_dev, bsum);
   return (int)cudaGetLastError();
 }
 
@@ -1301,7 +1296,7 @@ int launch_mask_offsets(const uint2* ranges, uint32_t num_tiles, uint32_t* words
                         cudaStream_t st) {
   if (num_tiles == 0) return 0;
   k_tile_words<<<grid_for(num_tiles, 256, 148 * 8), 256, 0, st>>>(ranges, num_tiles, words);
-  return launch_scan(words, nullptr, mask_off, num_tiles, nullptr, nullptr, nullptr, scratch, st);
+  return launch_scan(words, mask_off, num_tiles, nullptr, nullptr, scratch, st);
 }
 
 int launch_rect_counts(const uint4* rects, const uint32_t* depths, uint32_t n, uint32_t* counts, uint32_t* keys,
