@@ -65,10 +65,11 @@ def test_reference_arm_prints_on_rank0_only():
 
 
 def test_launch_count_matches_the_profiled_step():
-    """gpu_launches counts 64 kernels per chosen step on ring8_1m (35,392 tiles of 16 px over 8 views), the
-    number the ncu launch list of that step shows; the plain form launches per view."""
+    """gpu_launches counts 30 kernels per chosen step on ring8_1m (35,392 tiles of 16 px over 8 views), the
+    number a kernel trace of that step shows (test_gpu_launch_count.py counts a smaller step's); the plain form
+    launches per view."""
     import bench
-    assert bench.launches_per_step(35392, 8, "chosen") == 64
-    # two tile-sort passes for up to 65,536 tiles; a third beyond that
-    assert bench.launches_per_step(70000, 16, "chosen") == 64 + 2 * 5
-    assert bench.launches_per_step(35392, 8, "plain") == 8 * (38 + 2 + 1 + 1) + 5
+    assert bench.launches_per_step(35392, 8, "chosen") == 30
+    # two tile-sort passes for up to 65,536 tiles; a third beyond that, in both binnings
+    assert bench.launches_per_step(70000, 16, "chosen") == 30 + 2
+    assert bench.launches_per_step(8160, 1, "plain") == (13 + 2 + 1 + 2) + 6
