@@ -192,15 +192,16 @@ __device__ __forceinline__ W look_back(const W* col, uint32_t stride, uint32_t t
 // Against counting, scanning and scattering in five kernels per pass, each
 // pass reads its input once instead of twice, and a 32-bit sort takes 6
 // launches instead of 20. Whole 32-bit sorts of random keys in two arrays,
-// kernel time before and after: 16 thousand pairs 69 -> 37 us, 300 thousand
-// 76 -> 45, 1 million 97 -> 63, 4 million 182 -> 169, 12 million 585 -> 470; 32
-// million pairs of 16 bits 772 -> 614 us. Interleaved tile entries gain up to
-// 4 million (110 -> 87 us at 3.7 million) and lose beyond, also by chunks (below):
-// 8.6 million 164 -> 175 us, 33 million 545 -> 570. A tile takes 6 us by itself (chains of ballots, barriers and
-// L2 round trips), and the look-back grows with the tiles in flight: 2 blocks
-// of 512 threads per SM run the 4-million pass in 39 us, 3 blocks in 52, 6 of
-// 256 threads in 71, 8192-element tiles in 46 to 53; reading 16 or 32 tiles
-// back at once instead of 8, 40 and 43 us.
+// kernel time before and after: 16 thousand pairs 69 -> 33 us, 300 thousand
+// 76 -> 43, 1 million 97 -> 62, 4 million 182 -> 161, 12 million 585 -> 436; 32
+// million pairs of 16 bits 772 -> 566 us. Tile sorts of interleaved entries in
+// depth order, the larger ones by chunks (below): 2.9 million 85 -> 62 us, 8.6
+// million 164 -> 161, the 33 million of a 1080p frame 532 -> 516. A tile takes 6
+// us by itself (chains of ballots, barriers and L2 round trips), and the
+// look-back grows with the tiles in flight: 2 blocks of 512 threads per SM ran
+// the 4-million pass in 39 us (37.5 since match_digit has no branches), 3 blocks
+// in 52, 6 of 256 threads in 71, 8192-element tiles in 46 to 53; reading 16 or
+// 32 tiles back at once instead of 8, 40 and 43 us.
 constexpr int RS_THREADS = 512;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ROUNDS = RS_TILE / RS_THREADS;     // elements per thread per tile
@@ -209,16 +210,26 @@ constexpr int RS_CTAS = 2;                          // resident blocks per SM
 static_assert(RS_TILE == RS_THREADS * RS_ROUNDS && RS_ROUNDS % 2 == 0, "whole rounds");
 static_assert(RS_THREADS >= RS_BINS, "one thread per digit");
 
-// Lanes of the warp whose digit equals this lane's (multi-split by ballots).
+// Lanes of the warp whose digit (of nbits bits, nothing above them) equals this
+// lane's: multi-split by ballots, one per bit. Without a test for each bit:
+// with `if (b < nbits)` around it, every bit of every round was a branch
+// (156 million instructions a pass at 29 million pairs, 105 now; whole sorts of
+// 32 million pairs of 16 bits 627 -> 563 us, tile sorts of 2.9 million entries 71
+// -> 62). SHORT (tile ids, whose digits are often of 6 bits): the last two only
+// where they are used (29 million 252 -> 230 us for a pass of 6 bits; random keys
+// of 8 bits lose 2 % by it).
+template <bool SHORT>
 __device__ __forceinline__ uint32_t match_digit(uint32_t d, int nbits, uint32_t active) {
   uint32_t peers = active;
+  auto step = [&](int b) {
+    const uint32_t bal = __ballot_sync(FULL, (d >> b) & 1u);
+    peers &= bal ^ (((d >> b) & 1u) - 1u);
+  };
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    if (b < nbits) {
-      const uint32_t bit = (d >> b) & 1u;
-      const uint32_t bal = __ballot_sync(FULL, bit);
-      peers &= bit ? bal : ~bal;
-    }
+  for (int b = 0; b < 6; ++b) step(b);
+  if (!SHORT || nbits > 6) {
+    step(6);
+    step(7);
   }
   return peers;
 }
@@ -253,7 +264,7 @@ __device__ __forceinline__ uint64_t chunk_len(uint64_t n) {
 // reads it sequentially instead of through the permutation. PairIO's optional
 // value array (final pass only) receives the values alone.
 struct SplitIO {
-  static constexpr bool CHUNKS = false;
+  static constexpr bool CHUNKS = false, SHORT = false;
   const uint32_t* kin; const uint32_t* vin; uint32_t* kout; uint32_t* vout;
   const uint32_t* gsrc = nullptr; uint32_t* gdst = nullptr;
   SplitIO plain() const { SplitIO y = *this; y.gdst = nullptr; return y; }
@@ -268,7 +279,7 @@ struct SplitIO {
 };
 template <bool BY_CHUNKS>  // RC_MIN elements and more go by chunks
 struct PairIO {
-  static constexpr bool CHUNKS = BY_CHUNKS;
+  static constexpr bool CHUNKS = BY_CHUNKS, SHORT = true;
   const uint2* in; uint2* out;
   uint32_t* values = nullptr;
   PairIO plain() const { PairIO y = *this; y.values = nullptr; return y; }
@@ -444,7 +455,7 @@ __device__ __forceinline__ void chunk_pass(const IO& io, uint64_t n, int pass, i
       const bool valid = idx < tn;
       const uint32_t d = (e[r].x >> shift) & mask;
       const uint32_t act = __ballot_sync(FULL, valid);
-      const uint32_t peers = match_digit(d, nbits, act);
+      const uint32_t peers = match_digit<true>(d, nbits, act);
       uint32_t basev = 0;
       if (valid) basev = s_wh[warp][d];
       __syncwarp();
@@ -565,7 +576,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(IO io, uint64_t
       const bool valid = idx < tn;
       const uint32_t d = (e[r].x >> shift) & mask;
       const uint32_t act = __ballot_sync(FULL, valid);
-      const uint32_t peers = match_digit(d, nbits, act);
+      const uint32_t peers = match_digit<IO::SHORT>(d, nbits, act);
       uint32_t basev = 0;
       if (valid) basev = s_wh[warp][d];
       __syncwarp();
@@ -658,7 +669,7 @@ __global__ void __launch_bounds__(NT) k_rs_small(SplitIO io, int n, int passes, 
       const bool valid = idx < n;
       const uint32_t d = (e[r].x >> shift) & mask;
       const uint32_t act = __ballot_sync(FULL, valid);
-      const uint32_t peers = match_digit(d, nbits, act);
+      const uint32_t peers = match_digit<false>(d, nbits, act);
       uint32_t basev = 0;
       if (valid) basev = s_wh[warp][d];
       __syncwarp();
