@@ -365,18 +365,22 @@ void default_bwd_shape(gs_rasterizer* r) {
 // The backward's shape for a launch over `tiles` tiles. While neither
 // gs_set_launch_shapes nor the autotuner chose one, tiles of 16 pixels take 8
 // warps each when there are few (the longest tile decides) and 2 warps of 4
-// pixels a thread when there are many (throughput decides). Kernel time of
-// (64, 1) against (128, 2), on scenes of 16 and 100 thousand surfels spread
-// evenly and 40 and 200 thousand in clusters (whose longest tiles are far longer
-// than the mean): up to 3.2 tiles an SM 3 % slower to 25 % faster in every form.
-// One launch a tile: 4.0 an SM 216 and 224, 294 and 369, 376 and 365, 863 and 885
-// us for the four; 6.1 an SM 210 and 244, 281 and 431, 355 and 383, 663 and 835.
-// Persistent, heaviest tile first: 5.1 an SM 188 and 155, 216 and 252, 314 and
-// 262, 537 and 460; 7.8 an SM 201 and 292 (100 thousand), 425 and 477 (200).
-// (64, 4) against (128, 2), 100 and 200 thousand surfels, persistent and not: 24
-// an SM 290 and 259, 445 and 473, 497 and 493, 832 and 938; 31.5 an SM 428 and
-// 358, 621 and 558, 654 and 515, 1021 and 942; 55 an SM 474 and 382, 665 and 595,
-// 840 and 644, 1258 and 1095.
+// pixels a thread when there are many (throughput decides). How long the longest
+// tile is beside the mean is known on the device alone, so the lines are where
+// one shape wins on most scenes. Kernel times, us, (64, 1) / (128, 2):
+//   up to 3.2 tiles an SM, either form: 3 % slower to 25 % faster;
+//   one launch a tile, 16 and 100 thousand surfels spread evenly, 40 and 200
+//   thousand in clusters: 4.0 an SM 224/216, 369/294, 365/376, 885/863; 6.1 an SM
+//   244/210, 431/281, 383/355, 835/663;
+//   persistent, heaviest tile first, 4 to 200 thousand surfels, both kinds, ten
+//   framings: 4 to 5.1 an SM (76 runs) 8 % faster in the mean (clusters and frames
+//   the scene does not fill 7 to 28 % faster, evenly filled ones up to 31 %
+//   slower); 6.1 to 7.8 an SM (64 runs) 2 % in the mean and 22 of them slower, up
+//   to 32 %, so those stay with the shape that the form had before.
+// (128, 2) / (64, 4), 100 thousand spread evenly and 200 in clusters, persistent
+// and one launch a tile: 24 an SM 290/259, 445/473, 497/493, 832/938; 31.5 an SM
+// 428/358, 621/558, 654/515, 1021/942; 55 an SM 474/382, 665/595, 840/644,
+// 1258/1095.
 RasterShape bwd_shape(const gs_rasterizer* r, int tiles, bool persistent) {
   RasterShape s{r->bwd_batch, r->bwd_ppt};
   if (r->bwd_auto && r->tile == 16) {
