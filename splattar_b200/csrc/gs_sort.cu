@@ -239,18 +239,19 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d, int nbits, uint32_t 
 // and writing then overlap the next tile's loads, and there is one look-back
 // per chunk; but every pass after the first reads its keys once more to count
 // them. Tile sorts (two passes) of entries in depth order, counting included:
-// 2.9 million 71 us by look-back and 78 by chunks, 4.3 million 97 and 100,
-// 5.8 million 129 and 123, 8.6 million 186 and 175, 18 million 391 and 336, 29
-// million 601 and 514, the 33 million of a 1080p frame 681 and 570. With one
-// pass (up to 256 tiles) look-back stays ahead (5.8 million 96 and 131), and
-// so it does for two arrays (32 million pairs of 16 bits: 294 us a pass by
-// look-back; 341 by chunks, counted and scanned by kernels of their own).
+// 2.9 million 62 us by look-back and 74 by chunks, 5.8 million 113 and 115, 8.6
+// million 157 and 161, two frames of 9.5 million 349 and 318, 11.5 million 216
+// and 204, 18 million 341 and 317, 29 million 510 and 464, the 33 million of a
+// 1080p frame 580 and 516. With one pass (up to 256 tiles) look-back stays
+// ahead (5.8 million 96 and 131), and so it does for two arrays (32 million
+// pairs of 16 bits: 294 us a pass by look-back when chunks, counted and scanned
+// by kernels of their own, took 341).
 constexpr int RC_THREADS = RS_THREADS / 2, RC_WARPS = RC_THREADS / 32;
 constexpr int RC_TILE = RS_TILE / 2, RC_ROUNDS = RC_TILE / RC_THREADS;
 constexpr uint32_t RC_CHUNKS = 148 * RS_CTAS * 2;
 constexpr int RC_GROUP = 25;  // chunks whose counts are summed first
 constexpr int RC_GROUPS = (RC_CHUNKS + RC_GROUP - 1) / RC_GROUP;
-constexpr uint64_t RC_MIN = 5000000;
+constexpr uint64_t RC_MIN = 9000000;
 static_assert(RC_THREADS == RS_BINS, "one thread per digit");
 static_assert(RC_CHUNKS + RC_GROUPS <= RC_MIN / RS_TILE, "look-back words of the chunks and their groups");
 static_assert(RC_GROUPS <= RC_GROUP, "a look-back reads all groups at once");

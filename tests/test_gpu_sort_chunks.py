@@ -1,4 +1,4 @@
-"""Tile sorts of many entries (by chunks from 5 million on when two passes are
+"""Tile sorts of many entries (by chunks from 9 million on when two passes are
 needed): around that number, with one pass, and with every wait expiring at
 once. Integers: compared with a stable numpy sort by (tile, depth, item)."""
 import numpy as np
@@ -11,8 +11,8 @@ from test_gpu_project_binning import dev_to_host
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("total,tiles_x,tiles_y", [(4_999_999, 120, 68), (5_000_000, 120, 68), (5_000_001, 160, 90),
-                                                   (8_388_608, 32, 9), (6_000_003, 16, 16), (20_000_000, 257, 181)])
+@pytest.mark.parametrize("total,tiles_x,tiles_y", [(8_999_999, 120, 68), (9_000_000, 120, 68), (9_000_001, 160, 90),
+                                                   (9_699_328, 32, 9), (10_000_003, 16, 16), (20_000_000, 257, 181)])
 def test_binner_of_many_entries(total, tiles_x, tiles_y):
     """Items of `k` tiles in a row (the last one shorter), random places and depths with ties."""
     import torch
@@ -41,7 +41,7 @@ def test_binner_of_many_entries(total, tiles_x, tiles_y):
 
 
 def test_expired_waits_change_nothing_by_chunks():
-    n, sizes = 250000, [(1600, 900)] * 3
+    n, sizes = 400000, [(1600, 900)] * 3
     cams = ring_cameras(sizes)
     r = Rasterizer(n, 0, 0, 128 * n, max_views=3, max_pixels=sum(w * h for w, h in sizes))
     r.upload_scene(make_surfels(n, 7, True, 0, 0.1).scene_input())
@@ -51,7 +51,7 @@ def test_expired_waits_change_nothing_by_chunks():
         r.forward(cams, n)
         r.check()
         total = int(r.read("entry_count", 1)[0])
-        assert total > 5_000_000
+        assert total > 9_000_000
         got.append((r.read("ranges", 2 * 3 * 100 * 57), r.read("sorted_items", 2 * total)))
     for a in got[1:]:
         assert np.array_equal(a[0], got[0][0]) and np.array_equal(a[1], got[0][1])
