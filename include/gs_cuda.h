@@ -470,7 +470,7 @@ gs_status gs_exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, u
  * that must not pay an allocation's latency or implicit synchronisation, a
  * binding that forbids hidden allocations): it calls no allocator. Its
  * scratch is a fixed array in the library's device image sized for at most
- * 1,048,576 pairs (about 8.6 MB, held by every GPU that loads the library
+ * 1,048,576 pairs (about 8.9 MB, held by every GPU that loads the library
  * until exit); larger n returns GS_ERR_CAPACITY. The first call on a device
  * looks up that array's device address and keeps it for the process, so make
  * it before any stream capture, and do not call this entry point after
